@@ -16,7 +16,8 @@
 // Scoring: persistent CTAs copy the padded grid and the real scan into shared
 // memory once; each warp owns one hypothesis at a time and lanes cast
 // consecutive rays (neighbouring rays have similar lengths, which keeps the
-// DDA loops of a warp in step).  The DDA arithmetic is the reference's f32
+// DDA loops of a warp in step), stepped without branches (ray_chunk).  The DDA
+// arithmetic is the reference's f32
 // sequence (src/cuda/pf_kernels.cu:774-808) so per-ray distances agree bit
 // for bit; only the order of the CAER sum differs (lane-sequential, then an
 // xor butterfly).
@@ -45,7 +46,6 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kMaxSmem = 200 * 1024;
 
 GlHandle* as_gl(void* h) { return static_cast<GlHandle*>(h); }
 
@@ -107,25 +107,74 @@ __global__ void k_gl_gen_multi(int per_q, int n_yaw, int nfree,
 // (restarts are batched until kRestart lanes are free), so the warp is not
 // held by its longest ray.  The rays' crossing distances (ray_deltas: the
 // sincos and the divisions) are computed first with all lanes busy, so a
-// restart does neither; each ray's term |scan - raycast| then replaces them in
-// the ray's shared-memory slot, and the total is summed in the fixed
-// lane-sequential order
+// restart does neither; each ray's distance (or, with kPrune, its term |scan -
+// raycast|) then replaces them in the ray's shared-memory slot, and the total is
+// summed in the fixed lane-sequential order
 // (lane l adds rays l, l + 32, ..., then an xor butterfly), which does not
 // depend on the assignment.
 // With kPrune, the sum of the terms finished so far (any order) is compared
 // with `bound` at every restart and -1 is returned once it exceeds it; the
 // caller's bound includes a margin for the rounding difference between that
 // partial order and the final one.
-constexpr int kScoreThreads = 768;
-constexpr int kScoreWarps = kScoreThreads / 32;
+// A scorer block has at most 24 warps where two blocks share an SM (40 registers
+// a thread) and at most 32 where one block has it; score_plan chooses.
+constexpr int kPairThreads = 768;
+constexpr int kSoloThreads = 1024;
 // a launch keeps at least this many hypotheses per block on average, so a
 // small batch still reaches every SM without each block copying the grid
 // for a handful of warps
 constexpr int kMinScoreWarps = 8;
-constexpr int kChunk = 12;   // DDA steps between warp votes
-constexpr int kRestart = 8;  // free lanes that trigger a restart round
+// DDA steps between warp votes, and the free lanes that trigger a restart round
+// (40 000 hypotheses x 360 rays: 479 us at 12 steps, 471-472 at 16 to 24; 6 or
+// 10 lanes 472 and 474)
+constexpr int kChunk = 20;
+constexpr int kRestart = 8;
 
-template <bool kPrune>
+// The ray a lane of warp_caer holds: in the shared-memory form when the grid is
+// there, else stepping through global memory.
+template <bool kSmem>
+struct LaneRay;
+
+template <>
+struct LaneRay<true> {
+    SRay r;
+    __device__ __forceinline__ void none() { r.set_v(1u); }
+    __device__ __forceinline__ void begin(const unsigned char* g, const GridView& gv, int start,
+                                          float frx, float fry, float2 d) {
+        sray_init(r, gv.Wp, (unsigned)__cvta_generic_to_shared(g + start), frx, fry, d);
+    }
+    __device__ __forceinline__ bool ended() const { return r.hit() != 0u; }
+    template <int kN>
+    __device__ __forceinline__ void advance(const unsigned char*) {
+        ray_chunk<kN>(r);
+    }
+    __device__ __forceinline__ float result(const GridView&, int, float rmax, bool) const {
+        return sray_result(r, rmax);
+    }
+};
+
+template <>
+struct LaneRay<false> {
+    Ray r;
+    __device__ __forceinline__ void none() { r.v = 1u; }
+    __device__ __forceinline__ void begin(const unsigned char*, const GridView& gv, int start,
+                                          float frx, float fry, float2 d) {
+        ray_init_deltas(r, gv.Wp, start, frx, fry, d);
+    }
+    __device__ __forceinline__ bool ended() const { return r.v != 0u; }
+    template <int kN>
+    __device__ __forceinline__ void advance(const unsigned char* g) {
+#pragma unroll
+        for (int k = 0; k < kN; ++k)
+            if (r.v == 0u) ray_step(r, g);
+    }
+    __device__ __forceinline__ float result(const GridView& gv, int start, float rmax,
+                                            bool long_rays) const {
+        return ray_result(r, gv.Wp, start, rmax, long_rays);
+    }
+};
+
+template <bool kPrune, bool kSmem>
 __device__ __forceinline__ float warp_caer(const unsigned char* __restrict__ g,
                                            const GridView& gv, int Hp, float x,
                                            float y, float th,
@@ -151,41 +200,55 @@ __device__ __forceinline__ float warp_caer(const unsigned char* __restrict__ g,
         dirs[r] = ray_deltas(dx, dy, gv.res);
     }
     __syncwarp();
-    Ray ray;
+    LaneRay<kSmem> ray;
     int r = lane;
-    bool active = r < nrays;
-    ray.v = 1u;
-    if (active) ray_init_deltas(ray, gv.Wp, start, frx, fry, dirs[r]);
+    ray.none();
+    if (r < nrays) ray.begin(g, gv, start, frx, fry, dirs[r]);
+    unsigned act = nrays >= 32 ? ~0u : (1u << nrays) - 1u;  // lanes with a ray
     float lane_acc = 0.f;
     int next = 32;
     for (;;) {
-#pragma unroll
-        for (int k = 0; k < kChunk; ++k)
-            if (ray.v == 0u) ray_step(ray, g);
-        const unsigned done = __ballot_sync(~0u, active && ray.v != 0u);
-        const unsigned moving = __ballot_sync(~0u, active && ray.v == 0u);
-        if (moving != 0u && __popc(done) < kRestart) continue;
-        if (active && ray.v != 0u) {
-            const float t =
-                fabsf(sc[r] - ray_result(ray, gv.Wp, start, rmax, long_rays));
-            term[2 * r] = t;  // the ray's direction slot, no longer needed
-            lane_acc += t;
-            const int nr = next + __popc(done & lt);
-            if (nr < nrays) {
-                r = nr;
-                ray_init_deltas(ray, gv.Wp, start, frx, fry, dirs[r]);
-            } else {
-                active = false;
+        ray.template advance<kChunk>(g);
+        const unsigned done = __ballot_sync(~0u, ray.ended()) & act;
+        const int nd = __popc(done);
+        if (nd < kRestart && done != act) continue;
+        if (done >> lane & 1u) {
+            float t = ray.result(gv, start, rmax, long_rays);
+            if (kPrune) {
+                t = fabsf(sc[r] - t);
+                lane_acc += t;
             }
+            term[2 * r] = t;  // the ray's direction slot, no longer needed
+            r = next + __popc(done & lt);
+            if (r < nrays) ray.begin(g, gv, start, frx, fry, dirs[r]);
         }
-        next += __popc(done);
+        next += nd;
+        if (next > nrays) {  // no ray left for some of the lanes
+            act = __ballot_sync(~0u, r < nrays);
+            if (act == 0u) break;
+        }
         if (kPrune && warp_sum_f(lane_acc) > bound) return -1.0f;
-        if (!__any_sync(~0u, active)) break;
     }
     __syncwarp();
     float acc = 0.f;
-    for (int rr = lane; rr < nrays; rr += 32) acc += term[2 * rr];
+    for (int rr = lane; rr < nrays; rr += 32)
+        acc += kPrune ? term[2 * rr] : fabsf(sc[rr] - term[2 * rr]);
     return warp_sum_f(acc);
+}
+
+// Shared memory of the padded grid: ray_chunk may take kRayUnit - 1 steps past
+// the cell that ended a ray, so as many rows of slack lie on either side of it.
+__host__ __device__ __forceinline__ int grid_slack(int Wp) { return ((kRayUnit - 1) * Wp + 15) / 16 * 16; }
+
+// The padded grid copied into shared memory at smem; returns its first cell.
+__device__ __forceinline__ unsigned char* stage_padded(const GridView& gv, int grid_bytes,
+                                                       unsigned char* smem) {
+    unsigned char* g = smem + grid_slack(gv.Wp);
+    const int nv = grid_bytes / 16;
+    const uint4* src = reinterpret_cast<const uint4*>(gv.cells);
+    uint4* dst = reinterpret_cast<uint4*>(g);
+    for (int k = threadIdx.x; k < nv; k += blockDim.x) dst[k] = __ldg(&src[k]);
+    return g;
 }
 
 // Shared memory of the scorers: [padded grid (kSmem)] [scan] [per-warp ray
@@ -197,26 +260,36 @@ __device__ __forceinline__ void score_setup(const GridView& gv, int grid_bytes,
                                             const float*& sc, float*& term,
                                             float2*& dirs) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int gbytes = kSmem ? grid_bytes : 0;
-    float* s_scan = reinterpret_cast<float*>(smem + gbytes);
-    if (kSmem) {
-        const int nv = grid_bytes / 16;
-        const uint4* src = reinterpret_cast<const uint4*>(gv.cells);
-        uint4* dst = reinterpret_cast<uint4*>(smem);
-        for (int k = threadIdx.x; k < nv; k += blockDim.x) dst[k] = __ldg(&src[k]);
-    }
+    float* s_scan =
+        reinterpret_cast<float*>(smem + (kSmem ? grid_bytes + 2 * grid_slack(gv.Wp) : 0));
+    g = kSmem ? stage_padded(gv, grid_bytes, smem) : gv.cells;
     for (int k = threadIdx.x; k < nrays; k += blockDim.x) s_scan[k] = scan[k];
     __syncthreads();
-    g = kSmem ? smem : gv.cells;
     sc = s_scan;
     float2* slots = reinterpret_cast<float2*>(s_scan + ((nrays + 1) & ~1));
     dirs = slots + (size_t)(threadIdx.x >> 5) * nrays;
     term = reinterpret_cast<float*>(dirs);
 }
 
-// CAER of hypotheses [0, nh): one warp per hypothesis, static striding.
-template <bool kSmem>
-__global__ void __launch_bounds__(kScoreThreads, 2)
+// The hypotheses of a block (b, b + gridDim.x, ... of [0, n)) handed to its
+// warps as they finish: a hypothesis in a corner costs a fraction of one in
+// the open (40 000 hypotheses x 360 rays: 487 us with fixed shares, 472 so).
+// claim() returns n when none is left.
+struct WarpQueue {
+    unsigned* next;
+    int n;
+    __device__ __forceinline__ int claim() const {
+        unsigned k = 0;
+        if ((threadIdx.x & 31) == 0) k = atomicAdd(next, 1u);
+        k = __shfl_sync(~0u, k, 0);
+        const unsigned long long h = (unsigned long long)k * gridDim.x + blockIdx.x;
+        return h < (unsigned long long)n ? (int)h : n;
+    }
+};
+
+// CAER of hypotheses [0, nh): one warp per hypothesis.
+template <bool kSmem, int kT>
+__global__ void __launch_bounds__(kT, kT == kPairThreads ? 2 : 1)
     k_gl_score(GridView gv, int grid_bytes, const float* __restrict__ hyp,
                int nh, const float* __restrict__ scan, int nrays, float rmax,
                float span, float* __restrict__ caer) {
@@ -224,15 +297,13 @@ __global__ void __launch_bounds__(kScoreThreads, 2)
     const float* sc;
     float* term;
     float2* dirs;
-    score_setup<kSmem>(gv, grid_bytes, scan, nrays, g, sc, term, dirs);
+    __shared__ unsigned s_next;
+    if (threadIdx.x == 0) s_next = 0u;
+    score_setup<kSmem>(gv, grid_bytes, scan, nrays, g, sc, term, dirs);  // synchronises
+    const WarpQueue wq{&s_next, nh};
     const int Hp = gv.H + 2;
-    // hypotheses striped across the blocks first (warp w of block b takes
-    // b + w * gridDim.x, ...), so a batch smaller than the grid's warps is
-    // spread evenly over the SMs
-    const int gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    const int nw = gridDim.x * kScoreWarps;
-    for (int h = gw; h < nh; h += nw) {
-        const float c = warp_caer<false>(g, gv, Hp, hyp[3 * h], hyp[3 * h + 1],
+    for (int h = wq.claim(); h < nh; h = wq.claim()) {
+        const float c = warp_caer<false, kSmem>(g, gv, Hp, hyp[3 * h], hyp[3 * h + 1],
                                          hyp[3 * h + 2], sc, nrays, rmax, span,
                                          term, dirs, 0.f);
         if ((threadIdx.x & 31) == 0) caer[h] = c;
@@ -289,8 +360,8 @@ __device__ __forceinline__ float key_to_float(uint64_t key) {
 // so such a hypothesis ends above tau_f and can never enter the bottom-k.
 // The CAER of every hypothesis that is not dropped is the exhaustive
 // scorer's value; survivors (final key <= tau) are appended to cand.
-template <bool kSmem>
-__global__ void __launch_bounds__(kScoreThreads, 2)
+template <bool kSmem, int kT>
+__global__ void __launch_bounds__(kT, kT == kPairThreads ? 2 : 1)
     k_gl_score_pruned(GridView gv, int grid_bytes, const float* __restrict__ hyp,
                       int h0, int h1, const float* __restrict__ scan, int nrays,
                       float rmax, float span, float* __restrict__ caer,
@@ -299,19 +370,17 @@ __global__ void __launch_bounds__(kScoreThreads, 2)
     const float* sc;
     float* term;
     float2* dirs;
-    score_setup<kSmem>(gv, grid_bytes, scan, nrays, g, sc, term, dirs);
+    __shared__ unsigned s_next;
+    if (threadIdx.x == 0) s_next = 0u;
+    score_setup<kSmem>(gv, grid_bytes, scan, nrays, g, sc, term, dirs);  // synchronises
+    const WarpQueue wq{&s_next, h1 - h0};
     const int Hp = gv.H + 2;
     const unsigned long long tau = ctl->tau;
     const float tau_f = key_to_float(tau);
     const float bound = tau_f * (1.0f + 4.0f * (float)nrays * 5.9604645e-8f + 1e-6f);
     const int lane = threadIdx.x & 31;
-    // hypotheses striped across the blocks first (warp w of block b takes
-    // b + w * gridDim.x, ...), so a batch smaller than the grid's warps is
-    // spread evenly over the SMs
-    const int gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    const int nw = gridDim.x * kScoreWarps;
-    for (int h = h0 + gw; h < h1; h += nw) {
-        const float total = warp_caer<true>(g, gv, Hp, hyp[3 * h], hyp[3 * h + 1],
+    for (int h = h0 + wq.claim(); h < h1; h = h0 + wq.claim()) {
+        const float total = warp_caer<true, kSmem>(g, gv, Hp, hyp[3 * h], hyp[3 * h + 1],
                                             hyp[3 * h + 2], sc, nrays, rmax, span,
                                             term, dirs, bound);
         if (lane == 0) {
@@ -335,29 +404,25 @@ __global__ void __launch_bounds__(kScoreThreads, 2)
 // warp_caer as the single-query scorer, so every CAER equals the single-query
 // scorer's value bit for bit.  Shared memory: [padded grid (kSmem)] [per-warp
 // ray slots].
-template <bool kSmem>
-__global__ void __launch_bounds__(kScoreThreads, 2)
+template <bool kSmem, int kT>
+__global__ void __launch_bounds__(kT, kT == kPairThreads ? 2 : 1)
     k_gl_score_multi(GridView gv, int grid_bytes, const float* __restrict__ hyp,
                      int nh, int per_q, const float* __restrict__ scans, int nrays,
                      float rmax, float span, float* __restrict__ caer) {
     extern __shared__ __align__(16) unsigned char smem[];
-    if (kSmem) {
-        const int nv = grid_bytes / 16;
-        const uint4* src = reinterpret_cast<const uint4*>(gv.cells);
-        uint4* dst = reinterpret_cast<uint4*>(smem);
-        for (int k = threadIdx.x; k < nv; k += blockDim.x) dst[k] = __ldg(&src[k]);
-    }
+    __shared__ unsigned s_next;
+    if (threadIdx.x == 0) s_next = 0u;
+    const unsigned char* g = kSmem ? stage_padded(gv, grid_bytes, smem) : gv.cells;
     __syncthreads();
-    const unsigned char* g = kSmem ? smem : gv.cells;
-    float2* dirs = reinterpret_cast<float2*>(smem + (kSmem ? grid_bytes : 0)) +
+    const WarpQueue wq{&s_next, nh};
+    float2* dirs = reinterpret_cast<float2*>(
+                       smem + (kSmem ? grid_bytes + 2 * grid_slack(gv.Wp) : 0)) +
                    (size_t)(threadIdx.x >> 5) * nrays;
     float* term = reinterpret_cast<float*>(dirs);
     const int Hp = gv.H + 2;
-    const int gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    const int nw = gridDim.x * kScoreWarps;
-    for (int h = gw; h < nh; h += nw) {
+    for (int h = wq.claim(); h < nh; h = wq.claim()) {
         const float* sc = scans + (size_t)(h / per_q) * nrays;
-        const float c = warp_caer<false>(g, gv, Hp, hyp[3 * h], hyp[3 * h + 1],
+        const float c = warp_caer<false, kSmem>(g, gv, Hp, hyp[3 * h], hyp[3 * h + 1],
                                          hyp[3 * h + 2], sc, nrays, rmax, span, term,
                                          dirs, 0.f);
         if ((threadIdx.x & 31) == 0) caer[h] = c;
@@ -814,88 +879,83 @@ int ensure_scan(GlHandle* h, const float* scan, int nrays) {
     return 0;
 }
 
-template <bool kSmem>
-int score_grid_size(size_t smem) {
-    int per_sm = 0, sms = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gl_score<kSmem>,
-                                                  kScoreThreads, smem);
-    if (per_sm < 1) per_sm = 1;
-    return sms * per_sm;
+// Launch shape of a scorer with nrays ray slots per warp and nscan scan values
+// beside them.  The stepping is bound by issued instructions, so the shape with
+// the most warps on an SM is taken: two blocks of up to 24, else one of up to
+// 32 (20 011 hypotheses x 271 rays on 401 x 299 cells, which one block an SM
+// holds: 629 us at 24 warps before ray_chunk, 316 at 32 with it).  Where the padded grid leaves room for fewer than kMinSmemWarps it stays in
+// global memory and its cells come through L1; so it does where a ray could take
+// more than 8192 steps, which the shared-memory stepping does not count.
+constexpr int kSmBytes = 233472 - 2 * 1088;  // of an SM, less what each block reserves
+constexpr int kMaxSlotBytes = 200 * 1024;    // ray slots of 24 warps and the scan
+constexpr int kMinSmemWarps = 10;
+
+struct ScorePlan {
+    bool smem;
+    int warps, per_sm;
+    size_t bytes;
+};
+
+bool score_plan(const GlHandle* h, int nrays, int nscan, ScorePlan* p) {
+    const long long slot = (long long)sizeof(float2) * nrays;
+    const long long scan = (long long)sizeof(float) * ((nscan + 1) & ~1);
+    const long long grid = (long long)grid_bytes_padded(h) + 2 * grid_slack(h->Wp);
+    auto fit = [&](long long fixed, int per_sm, int most) {
+        return (int)std::max(0LL, std::min<long long>(most, (kSmBytes / per_sm - fixed) / slot));
+    };
+    const int solo = fit(grid + scan, 1, kSoloThreads / 32);
+    const int pair = fit(grid + scan, 2, kPairThreads / 32);
+    if (scan + slot * (kPairThreads / 32) > kMaxSlotBytes) {
+        set_error("pf_b200: %d rays need too much shared memory", nrays);
+        return false;
+    }
+    p->smem = std::max(solo, 2 * pair) >= kMinSmemWarps && h->Wp + h->Hp <= 8192;
+    if (p->smem) {
+        p->per_sm = 2 * pair > solo ? 2 : 1;
+        p->warps = p->per_sm == 2 ? pair : solo;
+        p->bytes = (size_t)(grid + scan + slot * p->warps);
+    } else {
+        const int w2 = fit(scan, 2, kPairThreads / 32), w1 = fit(scan, 1, kPairThreads / 32);
+        p->per_sm = w2 > 0 ? 2 : 1;
+        p->warps = w2 > 0 ? w2 : w1;
+        p->bytes = (size_t)(scan + slot * p->warps);
+    }
+    return true;
 }
 
-// Dynamic shared memory of a scorer launch; kSmem when the padded grid fits.
-size_t score_smem(const GlHandle* h, int nrays, bool* grid_in_smem) {
-    const size_t rest =
-        sizeof(float) * (size_t)((nrays + 1) & ~1) + sizeof(float2) * (size_t)nrays * kScoreWarps;
-    const size_t with_grid = (size_t)grid_bytes_padded(h) + rest;
-    *grid_in_smem = with_grid <= (size_t)kMaxSmem;
-    return *grid_in_smem ? with_grid : rest;
-}
+// Launch `kernel<kSmem, kT>` for n hypotheses under the plan.
+#define PFB_SCORE_LAUNCH(h, plan, n, kernel, ...)                                              \
+    do {                                                                                       \
+        const int grid_ = std::min((h)->sms * (plan).per_sm, ceil_div((n), kMinScoreWarps));   \
+        auto go_ = [&](auto* k_) -> int {                                                      \
+            /* one value for every plan: handles of other threads launch it too */             \
+            PFB_CK(cudaFuncSetAttribute(k_, cudaFuncAttributeMaxDynamicSharedMemorySize,       \
+                                        kSmBytes));                                            \
+            k_<<<grid_, 32 * (plan).warps, (plan).bytes, (h)->stream>>>(__VA_ARGS__);          \
+            PFB_KL();                                                                          \
+            return 0;                                                                          \
+        };                                                                                     \
+        const int rc_ = !(plan).smem          ? go_(kernel<false, kPairThreads>)               \
+                        : (plan).per_sm == 2 ? go_(kernel<true, kPairThreads>)                 \
+                                             : go_(kernel<true, kSoloThreads>);                \
+        if (rc_) return -1;                                                                    \
+    } while (0)
 
 int launch_score(GlHandle* h, int nrays, float rmax, float span) {
-    const int gb = grid_bytes_padded(h);
-    bool in_smem = false;
-    const size_t smem = score_smem(h, nrays, &in_smem);
-    if (smem > (size_t)kMaxSmem) {
-        set_error("pf_b200: pfgl_score: %d rays need too much shared memory", nrays);
-        return -1;
-    }
-    const GridView gv = grid_view(h);
-    const int warps_needed = h->nh;
-    if (in_smem) {
-        PFB_CK(cudaFuncSetAttribute(k_gl_score<true>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
-        int grid = score_grid_size<true>(smem);
-        grid = std::min(grid, ceil_div(warps_needed, kMinScoreWarps));
-        k_gl_score<true><<<grid, kScoreThreads, smem, h->stream>>>(
-            gv, gb, h->d_hyp, h->nh, h->d_scan, nrays, rmax, span, h->d_caer);
-    } else {
-        PFB_CK(cudaFuncSetAttribute(k_gl_score<false>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
-        int grid = score_grid_size<false>(smem);
-        grid = std::min(grid, ceil_div(warps_needed, kMinScoreWarps));
-        k_gl_score<false><<<grid, kScoreThreads, smem, h->stream>>>(
-            gv, gb, h->d_hyp, h->nh, h->d_scan, nrays, rmax, span, h->d_caer);
-    }
-    PFB_KL();
+    ScorePlan plan;
+    if (!score_plan(h, nrays, nrays, &plan)) return -1;
+    PFB_SCORE_LAUNCH(h, plan, h->nh, k_gl_score, grid_view(h), grid_bytes_padded(h), h->d_hyp,
+                     h->nh, h->d_scan, nrays, rmax, span, h->d_caer);
     return 0;
 }
 
 int launch_score_pruned(GlHandle* h, int h0, int h1, int nrays, float rmax,
                         float span) {
-    const int gb = grid_bytes_padded(h);
-    bool in_smem = false;
-    const size_t smem = score_smem(h, nrays, &in_smem);
-    if (smem > (size_t)kMaxSmem) {
-        set_error("pf_b200: pfgl_localize: %d rays need too much shared memory", nrays);
-        return -1;
-    }
-    const GridView gv = grid_view(h);
-    const int warps_needed = h1 - h0;
-    if (in_smem) {
-        PFB_CK(cudaFuncSetAttribute(k_gl_score_pruned<true>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
-        int grid = score_grid_size<true>(smem);
-        grid = std::min(grid, ceil_div(warps_needed, kMinScoreWarps));
-        k_gl_score_pruned<true><<<grid, kScoreThreads, smem, h->stream>>>(
-            gv, gb, h->d_hyp, h0, h1, h->d_scan, nrays, rmax, span, h->d_caer,
-            h->d_cand, h->d_ctl, h->cap_hyp);
-    } else {
-        PFB_CK(cudaFuncSetAttribute(k_gl_score_pruned<false>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
-        int grid = score_grid_size<false>(smem);
-        grid = std::min(grid, ceil_div(warps_needed, kMinScoreWarps));
-        k_gl_score_pruned<false><<<grid, kScoreThreads, smem, h->stream>>>(
-            gv, gb, h->d_hyp, h0, h1, h->d_scan, nrays, rmax, span, h->d_caer,
-            h->d_cand, h->d_ctl, h->cap_hyp);
-    }
-    PFB_KL();
+    ScorePlan plan;
+    if (!score_plan(h, nrays, nrays, &plan)) return -1;
+    PFB_SCORE_LAUNCH(h, plan, h1 - h0, k_gl_score_pruned, grid_view(h), grid_bytes_padded(h),
+                     h->d_hyp, h0, h1, h->d_scan, nrays, rmax, span, h->d_caer, h->d_cand,
+                     h->d_ctl, h->cap_hyp);
     return 0;
 }
 
@@ -1068,36 +1128,10 @@ int gl_localize_batch_enqueue(GlHandle* h, int nq, int per_q, int nrays, float r
     }
     const int nh = nq * per_q;
     h->nh = nh;
-    const int gb = grid_bytes_padded(h);
-    const size_t slots = sizeof(float2) * (size_t)nrays * kScoreWarps;
-    const bool in_smem = (size_t)gb + slots <= (size_t)kMaxSmem;
-    const size_t smem = in_smem ? gb + slots : slots;
-    if (smem > (size_t)kMaxSmem) {
-        set_error("pf_b200: %d rays need too much shared memory", nrays);
-        return -1;
-    }
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const GridView gv = grid_view(h);
-    if (in_smem) {
-        PFB_CK(cudaFuncSetAttribute(k_gl_score_multi<true>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gl_score_multi<true>,
-                                                      kScoreThreads, smem);
-        const int grid = std::min(sms * std::max(per_sm, 1), ceil_div(nh, kMinScoreWarps));
-        k_gl_score_multi<true><<<grid, kScoreThreads, smem, h->stream>>>(
-            gv, gb, h->d_hyp, nh, per_q, h->d_scans, nrays, rmax, span, h->d_caer);
-    } else {
-        PFB_CK(cudaFuncSetAttribute(k_gl_score_multi<false>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gl_score_multi<false>,
-                                                      kScoreThreads, smem);
-        const int grid = std::min(sms * std::max(per_sm, 1), ceil_div(nh, kMinScoreWarps));
-        k_gl_score_multi<false><<<grid, kScoreThreads, smem, h->stream>>>(
-            gv, gb, h->d_hyp, nh, per_q, h->d_scans, nrays, rmax, span, h->d_caer);
-    }
-    PFB_KL();
+    ScorePlan plan;
+    if (!score_plan(h, nrays, 0, &plan)) return -1;
+    PFB_SCORE_LAUNCH(h, plan, nh, k_gl_score_multi, grid_view(h), grid_bytes_padded(h), h->d_hyp,
+                     nh, per_q, h->d_scans, nrays, rmax, span, h->d_caer);
     h->caer_valid = true;
     k_select_small<true, false><<<nq, kSelThreads, 0, h->stream>>>(
         h->d_caer, nullptr, per_q, nullptr, k, h->d_keys, per_q);
@@ -1214,7 +1248,10 @@ void* pfgl_create(int W, int H, float res, float ox, float oy,
     const size_t gb = ((size_t)h->Wp * h->Hp + 15) / 16 * 16;
     bool ok = false;
     do {
-        if (cudaGetDevice(&h->dev) != cudaSuccess) break;
+        if (cudaGetDevice(&h->dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->dev) !=
+                cudaSuccess)
+            break;
         if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) !=
             cudaSuccess)
             break;
