@@ -127,15 +127,19 @@ __global__ void k_unpack(PlaneSet ps, int n, const float* pos3,
 
 PfHandle* as_pf(void* h) { return static_cast<PfHandle*>(h); }
 
-void drop_cycle_graph(PfHandle* h) {
-    if (h->cyc_exec) cudaGraphExecDestroy(h->cyc_exec);
-    if (h->cyc_graph) cudaGraphDestroy(h->cyc_graph);
-    h->cyc_exec = nullptr;
-    h->cyc_graph = nullptr;
+void drop_cycle_graph(PfHandle::CycleGraph& g) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    if (g.graph) cudaGraphDestroy(g.graph);
+    g.exec = nullptr;
+    g.graph = nullptr;
+}
+
+void drop_cycle_graphs(PfHandle* h) {
+    for (PfHandle::CycleGraph& g : h->cyc) drop_cycle_graph(g);
 }
 
 void free_particles(PfHandle* h) {
-    drop_cycle_graph(h);
+    drop_cycle_graphs(h);
     cudaFree(h->d_state[0]);
     cudaFree(h->d_state[1]);
     cudaFree(h->d_ll);
@@ -215,6 +219,10 @@ int wait_estimate(PfHandle* h) {
     h->stats.host_syncs += 1;
     h->est_inflight = false;
     h->est_valid = true;
+    if (h->last_obs_dev) {
+        h->dev_obs_mixed = h->dev_obs_mixed || !h->h_ctl->obs_cart;
+        h->dev_obs_cart = !h->dev_obs_mixed;
+    }
     return device_error(h);
 }
 
@@ -247,6 +255,12 @@ int ensure_stage(PfHandle* h) {
     return 0;
 }
 
+bool all_cartesian(const CObservation* obs, int nobs) {
+    int mode = 0;
+    for (int k = 0; k < nobs; ++k) mode |= obs[k].mode;
+    return mode == 0;
+}
+
 bool valid_handle(PfHandle* h) { return h != nullptr && h->n > 0; }
 
 // Everything a captured cycle depends on besides the per-cycle values.
@@ -269,13 +283,13 @@ void cycle_graph_key(const PfHandle* h, const PfcCycleParams* prm, long long k[1
 }
 
 int enqueue_cycle(PfHandle* h, const PredictArgs& pa, const CObservation* obs_dev,
-                  int nobs, const PfcCycleParams* prm, const CycleArgs* dargs);
+                  int nobs, bool cart, const PfcCycleParams* prm, const CycleArgs* dargs);
 
 // A fused cycle replayed from a CUDA graph (same kernels and arguments as the
 // direct launches; the per-cycle values come from d_cargs).  Used when there
 // are observations and per-kernel profiling is off.
 int run_cycle_graph(PfHandle* h, const PfcOdom* odom, const CObservation* obs_dev,
-                    int nobs, const PfcCycleParams* prm) {
+                    int nobs, bool cart, const PfcCycleParams* prm) {
     h->gen++;
     const int slot = h->cargs_pos;
     h->cargs_pos = (h->cargs_pos + 1) % PfHandle::kRing;
@@ -304,15 +318,16 @@ int run_cycle_graph(PfHandle* h, const PfcOdom* odom, const CObservation* obs_de
     h->stats.h2d_bytes += sizeof(CycleArgs);
     long long key[12];
     cycle_graph_key(h, prm, key);
-    if (h->cyc_exec && memcmp(key, h->graph_key, sizeof key) != 0) drop_cycle_graph(h);
-    if (!h->cyc_exec) {
+    PfHandle::CycleGraph& cg = h->cyc[weight_by_marks(h, nobs, cart) ? 1 : 0];
+    if (cg.exec && memcmp(key, cg.key, sizeof key) != 0) drop_cycle_graph(cg);
+    if (!cg.exec) {
         const long long l0 = h->stats.launches;
         const size_t d0 = h->stats.d2h_bytes;
         PFB_CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        const int rc = enqueue_cycle(h, a.pa, obs_dev, nobs, prm, h->d_cargs);
+        const int rc = enqueue_cycle(h, a.pa, obs_dev, nobs, cart, prm, h->d_cargs);
         cudaGraph_t g = nullptr;
         const cudaError_t e = cudaStreamEndCapture(h->stream, &g);
-        h->graph_kernels = (int)(h->stats.launches - l0);
+        cg.kernels = (int)(h->stats.launches - l0);
         h->stats.launches = l0;
         h->stats.d2h_bytes = d0;
         if (rc || e != cudaSuccess) {
@@ -320,13 +335,13 @@ int run_cycle_graph(PfHandle* h, const PfcOdom* odom, const CObservation* obs_de
             set_error("pf_b200: cycle graph capture failed: %s", cudaGetErrorString(e));
             return -1;
         }
-        h->cyc_graph = g;
-        PFB_CK(cudaGraphInstantiate(&h->cyc_exec, g, 0));
-        memcpy(h->graph_key, key, sizeof key);
+        cg.graph = g;
+        PFB_CK(cudaGraphInstantiate(&cg.exec, g, 0));
+        memcpy(cg.key, key, sizeof key);
     }
-    PFB_CK(cudaGraphLaunch(h->cyc_exec, h->stream));
+    PFB_CK(cudaGraphLaunch(cg.exec, h->stream));
     PFB_CK(cudaEventRecord(h->est_ev, h->stream));
-    h->stats.launches += h->graph_kernels;
+    h->stats.launches += cg.kernels;
     h->stats.d2h_bytes += sizeof(CycleCtl);
     h->prefix_valid = false;
     h->anc_valid = true;
@@ -337,10 +352,10 @@ int run_cycle_graph(PfHandle* h, const PfcOdom* odom, const CObservation* obs_de
 
 // One fused cycle; obs_dev points at device-resident observations.
 int run_cycle(PfHandle* h, const PfcOdom* odom, const CObservation* obs_dev,
-              int nobs, const PfcCycleParams* prm) {
+              int nobs, bool cart, const PfcCycleParams* prm) {
     if (flush_predict(h)) return -1;
     if (h->use_graph && nobs > 0 && !h->prof.on && h->d_cargs)
-        return run_cycle_graph(h, odom, obs_dev, nobs, prm);
+        return run_cycle_graph(h, odom, obs_dev, nobs, cart, prm);
     h->gen++;
     PredictArgs pa{};
     pa.enabled = 1;
@@ -355,7 +370,7 @@ int run_cycle(PfHandle* h, const PfcOdom* odom, const CObservation* obs_dev,
         if (launch_predict(h, pa)) return -1;
         if (set_wmode(h, WMODE_UNIFORM)) return -1;
     }
-    if (enqueue_cycle(h, pa, obs_dev, nobs, prm, nullptr)) return -1;
+    if (enqueue_cycle(h, pa, obs_dev, nobs, cart, prm, nullptr)) return -1;
     h->est_inflight = true;
     h->est_valid = false;
     return 0;
@@ -365,9 +380,9 @@ int run_cycle(PfHandle* h, const PfcOdom* odom, const CObservation* obs_dev,
 // of the control block.  With dargs (graph capture) the weighting pass runs
 // and reads its per-cycle values from dargs.
 int enqueue_cycle(PfHandle* h, const PredictArgs& pa, const CObservation* obs_dev,
-                  int nobs, const PfcCycleParams* prm, const CycleArgs* dargs) {
+                  int nobs, bool cart, const PfcCycleParams* prm, const CycleArgs* dargs) {
     if (nobs > 0 &&
-        launch_weight(h, pa, obs_dev, nobs, prm->sigma_r, prm->sigma_b, prm->gate,
+        launch_weight(h, pa, obs_dev, nobs, cart, prm->sigma_r, prm->sigma_b, prm->gate,
                       dargs))
         return -1;
     if (launch_cycle_decide(h, prm->resample_ess_ratio)) return -1;
@@ -651,7 +666,8 @@ int pfc_weight(void* hv, const CObservation* obs, int nobs, float sigma_r,
     if (stage_observations(h, obs, nobs)) return -1;
     PredictArgs pa = pending_args(h);
     h->pending_predict = false;
-    if (launch_weight(h, pa, h->d_obs, nobs, sigma_r, sigma_b, gate)) return -1;
+    h->last_obs_dev = false;
+    if (launch_weight(h, pa, h->d_obs, nobs, all_cartesian(obs, nobs), sigma_r, sigma_b, gate)) return -1;
     // materialise the weights with the resampler's prefixes now: the estimate
     // pass then reads them instead of re-deriving them from ll
     if (launch_weight_prefix(h, false, 0.0)) return -1;
@@ -777,7 +793,8 @@ int pfc_cycle(void* hv, const PfcOdom* odom, const CObservation* obs, int nobs,
     if (nobs > h->cap_obs) nobs = h->cap_obs;
     if (!obs) nobs = 0;
     if (nobs > 0 && stage_observations(h, obs, nobs)) return -1;
-    if (run_cycle(h, odom, h->d_obs, nobs, prm)) return -1;
+    h->last_obs_dev = false;
+    if (run_cycle(h, odom, h->d_obs, nobs, all_cartesian(obs, nobs), prm)) return -1;
     return finish_cycle(h, est_out);
 }
 
@@ -787,7 +804,8 @@ int pfc_cycle_device(void* hv, const PfcOdom* odom, const void* d_obs, int nobs,
     if (!valid_handle(h) || !odom || !prm) return -1;
     if (nobs > h->cap_obs) nobs = h->cap_obs;
     if (!d_obs) nobs = 0;
-    if (run_cycle(h, odom, static_cast<const CObservation*>(d_obs), nobs, prm))
+    h->last_obs_dev = nobs > 0;
+    if (run_cycle(h, odom, static_cast<const CObservation*>(d_obs), nobs, h->dev_obs_cart, prm))
         return -1;
     if (!est_out) return 0;
     return finish_cycle(h, est_out);
@@ -797,7 +815,7 @@ int pfc_set_graph(void* hv, int on) {
     PfHandle* h = as_pf(hv);
     if (!h) return -1;
     h->use_graph = on != 0;
-    if (!h->use_graph) drop_cycle_graph(h);
+    if (!h->use_graph) drop_cycle_graphs(h);
     return 0;
 }
 
@@ -895,7 +913,8 @@ int pfc_shard_finish(void* hv, const PfcCycleParams* prm, double* est_out) {
     if (h->shard_nobs > 0 ? launch_softmax_combine(h) : set_wmode(h, WMODE_UNIFORM))
         return -1;
     const PredictArgs none{};
-    if (enqueue_cycle(h, none, nullptr, 0, prm, nullptr)) return -1;
+    h->last_obs_dev = false;
+    if (enqueue_cycle(h, none, nullptr, 0, false, prm, nullptr)) return -1;
     h->est_inflight = true;
     h->est_valid = false;
     return finish_cycle(h, est_out);

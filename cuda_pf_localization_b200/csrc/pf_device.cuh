@@ -86,6 +86,24 @@ __device__ __forceinline__ GateConsts gate_consts(float sigma_r, float sigma_b,
     return g;
 }
 
+// Whether the gated Cartesian term r2 > cart_gate2 ? cart_out : RN(-r2 inv2rr)
+// is max(RN(-r2 inv2rr), cart_out) for every r2: the rounded product falls as
+// r2 grows, so it is when the product is not below cart_out at cart_gate2 and
+// not above it at the next float (true of most sigmas and gates).
+__device__ __forceinline__ bool cart_gate_is_max(const GateConsts& g) {
+    const float G = g.cart_gate2;
+    if (!(G > 0.0f) || !(G < 3.0e38f)) return false;
+    const float up = __uint_as_float(__float_as_uint(G) + 1u);
+    return __fmul_rn(-G, g.inv2rr) >= g.cart_out && __fmul_rn(-up, g.inv2rr) <= g.cart_out;
+}
+
+// max(a, b), NaN when a is NaN.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // x^2 + y^2 + z^2 as nvcc contracts the reference's squared residual:
 // fma(z, z, fma(x, x, y*y)).
 __device__ __forceinline__ float sq3(float x, float y, float z) {
@@ -323,16 +341,18 @@ __device__ __forceinline__ float2 block_softmax_partial(float acc0, bool v0,
 // Combine G block partials (executed by a whole block of kWThreads threads):
 // M = max of the block maxima, S = sum_b expf(m_b - M) * s_b in f32, each
 // reduced thread-strided, then by xor butterfly, then over warps in order.
-// The result is valid in every thread.
+// A larger block's further threads only wait.  The result is valid in every
+// thread.
 __device__ __forceinline__ float2 softmax_combine(const float2* part, int G) {
     __shared__ float s_d[kWThreads / 32];
     __shared__ float s_r;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid >= kWThreads) G = 0;
     float mx = -INFINITY;
 #pragma unroll 4
     for (int b = tid; b < G; b += kWThreads) mx = fmaxf(mx, __ldcg(&part[b].x));
     mx = warp_max_f(mx);
-    if (lane == 0) s_d[warp] = mx;
+    if (lane == 0 && tid < kWThreads) s_d[warp] = mx;
     __syncthreads();
     if (tid == 0) {
         float v = s_d[0];
@@ -349,7 +369,7 @@ __device__ __forceinline__ float2 softmax_combine(const float2* part, int G) {
     }
     sum = warp_sum_f(sum);
     __syncthreads();
-    if (lane == 0) s_d[warp] = sum;
+    if (lane == 0 && tid < kWThreads) s_d[warp] = sum;
     __syncthreads();
     if (tid == 0) {
         float S = 0.0f;
@@ -363,8 +383,9 @@ __device__ __forceinline__ float2 softmax_combine(const float2* part, int G) {
 // Gated log-likelihoods of two particles (p0,q0) and (p1,q1) against nobs
 // observations, staged kObsChunk at a time into shared memory (the whole
 // block takes part).  use_packed selects the packed f32x2 path for
-// all-Cartesian chunks; every path produces the reference's roundings.
-__device__ __forceinline__ void weight_two(
+// all-Cartesian chunks; every path produces the reference's roundings.  Returns
+// whether every observation kept was Cartesian.
+__device__ __forceinline__ bool weight_two(
     const CObservation* __restrict__ obs, int nobs, const float* __restrict__ lm,
     int lm_count, float sigma_r, float sigma_b, float gate, float3 p0, Quat q0,
     float3 p1, Quat q1, int use_packed, float& out0, float& out1) {
@@ -376,11 +397,13 @@ __device__ __forceinline__ void weight_two(
     const PackedPose pk = pack_pose(p0, qc0, p1, qc1);
     const float2 ninv = make_float2(-g.inv2rr, -g.inv2rr);
     float acc0 = 0.0f, acc1 = 0.0f;
+    bool cart = true;
     for (int c0 = 0; c0 < nobs; c0 += kObsChunk) {
         bool all_cart;
         __syncthreads();
         const int cn = stage_chunk(obs, lm, lm_count, c0, min(kObsChunk, nobs - c0),
                                    s_a, s_b, s_p, &all_cart);
+        cart = cart && all_cart;
         if (all_cart && use_packed) {
             float2 acc = make_float2(acc0, acc1);
             if (gate > 0.0f) {
@@ -430,6 +453,7 @@ __device__ __forceinline__ void weight_two(
     }
     out0 = acc0;
     out1 = acc1;
+    return cart;
 }
 
 // Attitude residual of q about qm as a canonical rotation vector

@@ -89,6 +89,8 @@ struct CycleCtl {
     // the estimate pass skipped sums 0..12 (a resample follows, the caller
     // said so with pfc_set_ess_hint); pfc_est_sums computes them on demand
     int est_partial;
+    // whether every observation of the last weighting was Cartesian
+    int obs_cart;
 };
 
 // Fixed-point image of a normalised f32 weight: round-to-nearest-even of
@@ -239,6 +241,10 @@ struct PfHandle {
     double* d_part = nullptr;           // per-block partials (max over uses)
     int part_cap = 0;                   // doubles in d_part
     unsigned long long* d_part_u64 = nullptr;  // per-block integer partials
+    // observations in device memory, which the host has not seen: Cartesian in the
+    // last cycle that was waited for (0 until then), never again after a cycle
+    // that was not
+    bool dev_obs_cart = false, dev_obs_mixed = false, last_obs_dev = false;
     bool prefix_valid = false;  // ctl w_total_fx and d_wprefix describe the
                                 // current weights
     unsigned* d_done = nullptr;         // last-block counters
@@ -284,10 +290,14 @@ struct PfHandle {
     cudaEvent_t cargs_ev[kRing] = {};
     int cargs_pos = 0;
     bool use_graph = true;
-    cudaGraph_t cyc_graph = nullptr;
-    cudaGraphExec_t cyc_exec = nullptr;
-    long long graph_key[12] = {};
-    int graph_kernels = 0;
+    // one for each weighting kernel, so a change of the observation count that
+    // changes the kernel does not capture again
+    struct CycleGraph {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        long long key[12] = {};
+        int kernels = 0;
+    } cyc[2];
 
     // accounting: kernels launched, bytes copied host<->device, host syncs
     PfcStats stats{};
@@ -349,8 +359,12 @@ int launch_reinit_poses(PfHandle* h, const float* d_poses, int k, float z,
 int launch_predict(PfHandle* h, const PredictArgs& pa);
 // Weighting (optionally fused with a deferred predict): writes ll, block
 // (max, sumexp) partials and the finalised M, S into the control block.
+// Whether launch_weight rotates every landmark once (a kernel of its own, so a
+// captured cycle holds for one answer).  cart: all observations are taken to be
+// Cartesian (a wrong guess costs time only).
+bool weight_by_marks(const PfHandle* h, int nobs, bool cart);
 int launch_weight(PfHandle* h, const PredictArgs& pa, const CObservation* d_obs,
-                  int nobs, float sigma_r, float sigma_b, float gate,
+                  int nobs, bool cart, float sigma_r, float sigma_b, float gate,
                   const CycleArgs* dargs = nullptr);
 // A sharded filter's slice (predict + weighting, block partials kept for the
 // exchange), and the softmax combine over every rank's partials after it.

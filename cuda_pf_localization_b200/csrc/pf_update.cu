@@ -8,7 +8,11 @@
 // so M = max ll and S = sum exp(ll - M) are deterministic.
 #include <math.h>
 
+
+#include <algorithm>
+
 #include "pf_device.cuh"
+#include "pf_marks.cuh"
 
 namespace pfb {
 
@@ -161,8 +165,9 @@ __global__ void __launch_bounds__(kWThreads, 5)
         }
     }
     float acc0, acc1;
-    weight_two(obs, nobs, lm, lm_count, sigma_r, sigma_b, gate, p0, q0, p1, q1,
-               use_packed, acc0, acc1);
+    const bool cart = weight_two(obs, nobs, lm, lm_count, sigma_r, sigma_b, gate, p0, q0, p1, q1,
+                                 use_packed, acc0, acc1);
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->obs_cart = cart ? 1 : 0;
     if (v0) ll[i0] = acc0;
     if (v1) ll[i1] = acc1;
     if (kShard) {
@@ -173,7 +178,264 @@ __global__ void __launch_bounds__(kWThreads, 5)
     }
 }
 
+// Softmax partial of a 256-particle tile by one warp: block_softmax_partial's
+// maximum and its sums, warp by warp of that block, in its order.
+__device__ __forceinline__ float2 tile_softmax_partial(const float* s_ll, int count) {
+    const int lane = threadIdx.x & 31;
+    float a[kWThreads / 32], b[kWThreads / 32];
+    float m = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < kWThreads / 32; ++w) {
+        const int i0 = 32 * w + lane, i1 = i0 + kWThreads;
+        a[w] = i0 < count ? s_ll[i0] : -INFINITY;
+        b[w] = i1 < count ? s_ll[i1] : -INFINITY;
+        m = fmaxf(m, fmaxf(a[w], b[w]));
+    }
+    const float bm = warp_max_f(m);
+    float sb = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kWThreads / 32; ++w) {
+        const int i0 = 32 * w + lane, i1 = i0 + kWThreads;
+        const float e = __fadd_rn(i0 < count ? expf(__fsub_rn(a[w], bm)) : 0.0f,
+                                  i1 < count ? expf(__fsub_rn(b[w], bm)) : 0.0f);
+        sb = __fadd_rn(sb, warp_sum_f(e));
+    }
+    return make_float2(bm, sb);
+}
+
+// Any observations, a particle per thread: k_weight_marks' way with bearings.
+template <bool kPredict>
+__device__ __noinline__ void weight_tiles(MarksSmem& sm, const Planes& s, int n, uint64_t seed,
+                                          const PredictArgs& pa,
+                                          const CObservation* __restrict__ obs, int nobs,
+                                          const float* __restrict__ lm, int lm_count,
+                                          float sigma_r, float sigma_b, float gate,
+                                          float* __restrict__ ll, float2* part) {
+    constexpr int kTile = kMTile;
+    const GateConsts g = gate_consts(sigma_r, sigma_b, gate);
+    const int tid = threadIdx.x;
+    __syncthreads();
+    if (tid < nobs) {
+        const CObservation o = obs[tid];
+        const bool keep = o.id >= 0 && o.id < lm_count;
+        const float* l = lm + 3 * (keep ? o.id : 0);
+        sm.rec[2 * tid] = make_float4(l[0], l[1], l[2],
+                                      __int_as_float(!keep ? 0 : o.mode == 0 ? 1 : 2));
+        sm.rec[2 * tid + 1] = make_float4(o.dx, o.dy, o.dz, o.range);
+    }
+    __syncthreads();
+    for (int tile = blockIdx.x; tile * kTile < n; tile += gridDim.x) {
+        const int i = tile * kTile + tid;
+        if (tid < kTile && i < n) {
+            float3 p;
+            Quat q;
+            load_pose(s, i, p, q);
+            if (kPredict) {
+                apply_predict(pa, seed, i, p, q);
+                store_pose(s, i, p, q);
+            }
+            const Quat qc = q_conjugate(q);
+            float acc = 0.0f;
+            for (int k = 0; k < nobs; ++k) {
+                const float4 a = sm.rec[2 * k];
+                const int kind = __float_as_int(a.w);
+                if (kind != 0) obs_loglik(g, p, qc, a, sm.rec[2 * k + 1], kind, acc);
+            }
+            ll[i] = acc;
+            sm.ll[0][0][tid] = acc;
+        }
+        __syncthreads();
+        if (tid < 32) {
+            const float2 pb = tile_softmax_partial(sm.ll[0][0], min(kTile, n - tile * kTile));
+            if (tid == 0) part[tile] = pb;
+        }
+        __syncthreads();
+    }
+}
+
+// k_weight with every landmark rotated once per particle (pf_marks.cuh), for up to
+// kMObs Cartesian observations of up to kMMarks landmarks: one persistent block
+// per SM over the same 256-particle tiles, so the log-likelihoods and the softmax
+// partials are k_weight's to the bit.  The groups take the block's tiles as they
+// finish; the markers predict their first tile themselves, the scouts the others.
+// Observations that are not all Cartesian (a device buffer whose contents the host
+// has not seen) take weight_tiles.
+template <bool kPredict>
+__global__ void __launch_bounds__(kMThreads, 1)
+    k_weight_marks(PlaneSet ps, int n, uint64_t seed, PredictArgs pa,
+                   const CObservation* __restrict__ obs, int nobs, const float* __restrict__ lm,
+                   int lm_count, float sigma_r, float sigma_b, float gate,
+                   float* __restrict__ ll, float2* part, unsigned* done, CycleCtl* ctl,
+                   const CycleArgs* ca) {
+    extern __shared__ __align__(16) unsigned char marks_smem[];
+    MarksSmem& sm = *reinterpret_cast<MarksSmem*>(marks_smem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_wait();
+    if (warp == 0) {
+        umma::tmem_alloc(&sm.tmem, kMMarks * kMColumns);
+        umma::tmem_relinquish();
+    }
+    umma::tc_fence_before();
+    if (ca) {  // graph replay: this cycle's values
+        pa = ca->pa;
+        obs = ca->obs;
+        nobs = ca->nobs;
+    }
+    const Planes s = pick_planes(ps, ctl->live);
+    marks_build(sm, obs, min(nobs, kMObs), lm, lm_count);  // synchronises
+    umma::tc_fence_after();
+    const int ntiles = (n + kMTile - 1) / kMTile;
+    const bool marker = warp < kMGroups * kMMarkers;
+    const int group = marker ? warp / kMMarkers : (warp - kMGroups * kMMarkers) / kMScouts;
+    const int w = marker ? warp % kMMarkers : (warp - kMGroups * kMMarkers) % kMScouts;
+    bool ok = true;
+    if (blockIdx.x == 0 && tid == 0) ctl->obs_cart = sm.all_cart;
+    if (!sm.all_cart) {
+        weight_tiles<kPredict>(sm, s, n, seed, pa, obs, min(nobs, kMObs), lm, lm_count, sigma_r,
+                               sigma_b, gate, ll, part);
+    } else if (marker) {
+        const GateConsts g = gate_consts(sigma_r, sigma_b, gate);
+        const bool gate_max = cart_gate_is_max(g);
+        const SharedMarks in_shared{smem_addr(&sm.pred[w][0][0][lane])};
+        const TensorMarks in_tensor{sm.tmem + ((uint32_t)(32 * w) << 16)};
+        int tile = blockIdx.x + group * gridDim.x;
+        for (int k = 0; tile >= 0 && tile < ntiles; ++k) {
+            const int l = w * kMUnit + 2 * lane, i = tile * kMTile + l;
+            float3 p[2];
+            Quat q[2];
+            if (k == 0) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    p[h] = make_float3(0.f, 0.f, 0.f);
+                    q[h] = {1.f, 0.f, 0.f, 0.f};
+                    if (i + h < n) {
+                        load_pose(s, i + h, p[h], q[h]);
+                        if (kPredict) {
+                            apply_predict(pa, seed, i + h, p[h], q[h]);
+                            store_pose(s, i + h, p[h], q[h]);
+                        }
+                    }
+                }
+            } else {
+                auto two = [&](int c) {
+                    return *reinterpret_cast<const float2*>(&sm.pose[group][c][l]);
+                };
+                const float2 x = two(0), y = two(1), z = two(2);
+                const float2 qw = two(3), qx = two(4), qy = two(5), qz = two(6);
+                marks_arrive(&sm.taken[group]);
+                p[0] = make_float3(x.x, y.x, z.x);
+                p[1] = make_float3(x.y, y.y, z.y);
+                q[0] = {qw.x, qx.x, qy.x, qz.x};
+                q[1] = {qw.y, qx.y, qy.y, qz.y};
+            }
+            const PackedPose pk = pack_pose(p[0], q_conjugate(q[0]), p[1], q_conjugate(q[1]));
+            const float2 acc = group == 0 ? marks_unit(sm, in_tensor, g, gate_max, pk)
+                                          : marks_unit(sm, in_shared, g, gate_max, pk);
+            const int b = k & 1, phase = (k >> 1) & 1;
+            if (k > 1 && !marks_wait(sm, &sm.summed[group][b], phase ^ 1)) {
+                ok = false;
+                break;
+            }
+            *reinterpret_cast<float2*>(&sm.ll[group][b][l]) = acc;
+            if (i + 1 < n)
+                *reinterpret_cast<float2*>(&ll[i]) = acc;
+            else if (i < n)
+                ll[i] = acc.x;
+            marks_arrive(&sm.scored[group][b]);
+            ok = marks_wait(sm, &sm.ready[group], k & 1);
+            if (!ok) break;
+            tile = *const_cast<volatile int*>(&sm.tile[group]);
+        }
+    } else {
+        int tile = blockIdx.x + group * gridDim.x;
+        for (int k = 0; tile >= 0 && tile < ntiles; ++k) {
+            // the group works on tile k; prepare tile k + 1
+            if (k > 0 && !(ok = marks_wait(sm, &sm.taken[group], (k - 1) & 1))) break;
+            if (w == 0) {
+                if (lane == 0) {
+                    const int next = atomicAdd(&sm.next, 1) * (int)gridDim.x + blockIdx.x;
+                    sm.tile[group] = next < ntiles ? next : -1;
+                }
+                marks_arrive(&sm.claimed[group]);
+            }
+            if (!(ok = marks_wait(sm, &sm.claimed[group], k & 1))) break;
+            const int next = *const_cast<volatile int*>(&sm.tile[group]);
+            for (int l = 32 * w + lane; next >= 0 && l < kMTile; l += 32 * kMScouts) {
+                const int i = next * kMTile + l;
+                float3 p = make_float3(0.f, 0.f, 0.f);
+                Quat q = {1.f, 0.f, 0.f, 0.f};
+                if (i < n) {
+                    load_pose(s, i, p, q);
+                    if (kPredict) {
+                        apply_predict(pa, seed, i, p, q);
+                        store_pose(s, i, p, q);
+                    }
+                }
+                const float v[7] = {p.x, p.y, p.z, q.w, q.x, q.y, q.z};
+#pragma unroll
+                for (int c = 0; c < 7; ++c) sm.pose[group][c][l] = v[c];
+            }
+            marks_arrive(&sm.ready[group]);
+            if (w == 0) {
+                const int b = k & 1;
+                if (!(ok = marks_wait(sm, &sm.scored[group][b], (k >> 1) & 1))) break;
+                const float2 pb =
+                    tile_softmax_partial(sm.ll[group][b], min(kMTile, n - tile * kMTile));
+                if (lane == 0) part[tile] = pb;
+                marks_arrive(&sm.summed[group][b]);
+            }
+            tile = next;
+        }
+    }
+    if (!ok && lane == 0) atomicOr(&ctl->err, ERR_SPIN_TIMEOUT);
+    umma::tc_fence_before();
+    __threadfence();
+    __shared__ bool s_last;
+    __syncthreads();
+    if (warp == 0) {
+        umma::tc_fence_after();
+        umma::tmem_dealloc(sm.tmem, kMMarks * kMColumns);
+    }
+    if (tid == 0) s_last = (atomicAdd(done, 1u) == gridDim.x - 1);
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const float2 ms = softmax_combine(part, ntiles);
+    if (tid == 0) {
+        softmax_commit(ms, ctl);
+        *done = 0u;
+    }
+}
+
+constexpr int kMarksGrid = 148;
+
+template <bool kPredict>
+int launch_marks(PfHandle* h, const PredictArgs& pa, const CObservation* d_obs, int nobs,
+                 float sigma_r, float sigma_b, float gate, const CycleArgs* dargs) {
+    PFB_CK(cudaFuncSetAttribute(k_weight_marks<kPredict>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)sizeof(MarksSmem)));
+    const int grid = std::min(ceil_div(h->n, 2 * kWThreads), kMarksGrid);
+    PFB_CK(launch_pdl(k_weight_marks<kPredict>, grid, kMThreads, sizeof(MarksSmem), h->stream,
+                      plane_set(h), h->n, h->seed, pa, d_obs, nobs, h->d_lm, h->lm_count, sigma_r,
+                      sigma_b, gate, h->d_ll, reinterpret_cast<float2*>(h->d_part), h->d_done + 0,
+                      h->d_ctl, dargs));
+    return 0;
+}
+
 }  // namespace
+
+// Rotating a landmark once saves 21 of an observation's 29 operations for all but
+// its first, and costs a block the set-up and two tiles' latency.  k_weight and
+// k_weight_marks measured (us, particles x landmarks / observations): 1M x 64/256
+// 283 and 194, 1M x 12/128 160 and 109, 1M x 32/96 131 and 113, 1M x 32/64 100 and
+// 100, 200k x 32/128 45 and 41, 100k x 64/256 45 and 43, 100k x 64/192 38 and 39,
+// 200k x 64/128 45 and 47.
+bool weight_by_marks(const PfHandle* h, int nobs, bool cart) {
+    return cart && h->weight_variant == 0 && h->lm_count > 0 && h->lm_count <= kMMarks &&
+           nobs <= kMObs && nobs >= 96 && nobs >= 2 * h->lm_count &&
+           (long long)h->n * (nobs - h->lm_count) >= 16000000;
+}
 
 int launch_reinit(PfHandle* h, const float p0[3], const float q0[4],
                   const float pstd[3], const float rstd[3]) {
@@ -210,12 +472,16 @@ int launch_predict(PfHandle* h, const PredictArgs& pa) {
 }
 
 int launch_weight(PfHandle* h, const PredictArgs& pa, const CObservation* d_obs,
-                  int nobs, float sigma_r, float sigma_b, float gate,
+                  int nobs, bool cart, float sigma_r, float sigma_b, float gate,
                   const CycleArgs* dargs) {
     const int grid = ceil_div(h->n, 2 * kWThreads);
     float2* part = reinterpret_cast<float2*>(h->d_part);
     KernelScope ks(h, KK_WEIGHT);
-    if (pa.enabled) {
+    if (weight_by_marks(h, nobs, cart)) {
+        if (pa.enabled ? launch_marks<true>(h, pa, d_obs, nobs, sigma_r, sigma_b, gate, dargs)
+                       : launch_marks<false>(h, pa, d_obs, nobs, sigma_r, sigma_b, gate, dargs))
+            return -1;
+    } else if (pa.enabled) {
         PFB_CK(launch_pdl(k_weight<true, false>, grid, kWThreads, 0, h->stream, plane_set(h),
                           h->n, h->seed, pa, d_obs, nobs, h->d_lm, h->lm_count,
                           sigma_r, sigma_b, gate, h->d_ll, part, h->d_done + 0,
