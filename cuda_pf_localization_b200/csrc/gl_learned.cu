@@ -94,68 +94,131 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
     return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// Epilogue of 32 consecutive columns [col0, col0 + 32) of one output row.
+// Epilogue of one warp's 32 rows x 32 columns at (row0, col0): lane l arrives with
+// row row0 + l.  The chunk passes through 4 KiB of shared memory and leaves in
+// 16-byte pieces, of which four lanes (bf16) or eight (f32) fill a 64- or 128-byte
+// line segment of the output, and of the transposed one.  Stored from the registers
+// as they are, each lane writes 16 bytes of its own row at a time, half a sector,
+// and two bytes a column of the transpose: the epilogue, not the MMAs, then bounds a
+// tile (26 of a launch's 38 thousand cycles).  Training step, so stored and as here:
+// 389 and 355 us at a batch of 8192, 210 and 200 at 2048, 181 and 172 at 512 (CTA
+// pairs with 256 x 256 tiles were slower than this, 364 at 8192).
+// m: the chunk's mask words (relu' gating).
+constexpr int kStagedBytes = 4096;  // of an epilogue warp
 template <int EPI>
-__device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[32], int row,
-                                               int col0, const float* bias,
-                                               const EpiArgs& ep) {
-    float v[32];
+__device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[32], const uint4 (&m)[4],
+                                               int row0, int col0, const float* bias,
+                                               const EpiArgs& ep, unsigned char* stage) {
+    const int lane = threadIdx.x & 31;
+    uint4* rows = reinterpret_cast<uint4*>(stage);  // [row][pieces], swizzled
+    if constexpr (EPI == EPI_F32 || EPI == EPI_BIAS_F32) {
+        const float s = EPI == EPI_F32 ? ep.scale : 1.0f;
+        auto value = [&](int j) {
+            float v = __uint_as_float(r[j]);
+            if (EPI == EPI_BIAS_F32) v += bias[j];
+            return __float_as_uint(v * s);
+        };
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-    if (EPI == EPI_RELU_BF16 || EPI == EPI_BIAS_F32) {
+        for (int q = 0; q < 8; ++q)
+            rows[8 * lane + (q ^ (lane & 7))] = make_uint4(value(4 * q), value(4 * q + 1),
+                                                           value(4 * q + 2), value(4 * q + 3));
+        __syncwarp();
+        const int line = lane >> 3, piece = lane & 7;
+        float* out = reinterpret_cast<float*>(ep.out) + (size_t)row0 * ep.ldo + col0 + 4 * piece;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] += bias[j];  // shared memory
-    }
-    if (EPI == EPI_RELU_BF16) {
+        for (int i = 0; i < 8; ++i) {
+            const int x = 4 * i + line;
+            *reinterpret_cast<uint4*>(out + (size_t)x * ep.ldo) = rows[8 * x + (piece ^ (x & 7))];
+        }
+    } else {
+        uint32_t w[16];  // columns (2k, 2k + 1) of row `lane`
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
-    }
-    if (EPI == EPI_DRELU_BF16) {
-        const uint4* mp = reinterpret_cast<const uint4*>(
-            ep.mask + (size_t)row * ep.ldm + col0);
+        for (int k = 0; k < 16; ++k) {
+            float a = __uint_as_float(r[2 * k]), b = __uint_as_float(r[2 * k + 1]);
+            if (EPI == EPI_RELU_BF16) {
+                a = fmaxf(a + bias[2 * k], 0.0f);
+                b = fmaxf(b + bias[2 * k + 1], 0.0f);
+            } else {
+                const uint4 u = m[k / 4];
+                const uint32_t x = k % 4 == 0 ? u.x : k % 4 == 1 ? u.y : k % 4 == 2 ? u.z : u.w;
+                // relu'(z) = 1 exactly when the stored activation is > 0
+                if ((int)(short)(x & 0xFFFFu) <= 0) a = 0.0f;
+                if ((int)(short)(x >> 16) <= 0) b = 0.0f;
+            }
+            w[k] = pack_bf16x2(a, b);
+        }
+        uint32_t* cols = reinterpret_cast<uint32_t*>(stage + 2048);  // [column][16 row pairs]
+        const int sw = (lane >> 1) & 3;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint4 u = mp[q];
-            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+        for (int q = 0; q < 4; ++q)
+            rows[4 * lane + (q ^ sw)] =
+                make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+        if (ep.outT) {
+            // even lanes take the even columns of their row and the next, odd lanes
+            // the odd ones
+            const bool odd = lane & 1;
 #pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                // relu'(z) = 1 exactly when the stored activation is > 0:
-                // a bf16 bit pattern in [1, 0x7fff].
-                const int lo = (int)(short)(w[t] & 0xFFFFu);
-                const int hi = (int)(short)(w[t] >> 16);
-                if (lo <= 0) v[q * 8 + 2 * t] = 0.0f;
-                if (hi <= 0) v[q * 8 + 2 * t + 1] = 0.0f;
+            for (int k = 0; k < 16; ++k) {
+                const uint32_t o = __shfl_xor_sync(~0u, w[k], 1);
+                cols[(2 * k + (lane & 1)) * 16 + (lane >> 1)] =
+                    odd ? __byte_perm(o, w[k], 0x7632) : __byte_perm(w[k], o, 0x5410);
+            }
+        }
+        __syncwarp();
+        const int line = lane >> 2, piece = lane & 3;
+        bf16* out = reinterpret_cast<bf16*>(ep.out) + (size_t)row0 * ep.ldo + col0 + 8 * piece;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int x = 8 * i + line;
+            *reinterpret_cast<uint4*>(out + (size_t)x * ep.ldo) =
+                rows[4 * x + (piece ^ ((x >> 1) & 3))];
+        }
+        if (ep.outT) {
+            bf16* outT = reinterpret_cast<bf16*>(ep.outT) + (size_t)col0 * ep.ldt + row0 + 8 * piece;
+            const uint4* c4 = reinterpret_cast<const uint4*>(cols);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int x = 8 * i + line;
+                *reinterpret_cast<uint4*>(outT + (size_t)x * ep.ldt) = c4[4 * x + piece];
             }
         }
     }
-    if (EPI == EPI_BIAS_F32 || EPI == EPI_F32) {
-        const float s = EPI == EPI_F32 ? ep.scale : 1.0f;
-        float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(ep.out) +
-                                              (size_t)row * ep.ldo + col0);
+    __syncwarp();  // the stage is reused
+}
+
+// One epilogue warp's chunks part, part + kPerQ, ... of its 32 rows of a tile, with
+// the mask of each loaded while the one before is stored.  last(): called once the
+// accumulator has been read.
+template <int EPI, int kChunks, int kPerQ, class Last>
+__device__ __forceinline__ void epilogue_tile(uint32_t trow, int row0, int n0, int part,
+                                              const EpiArgs& ep, unsigned char* stage,
+                                              Last last) {
+    const int lane = threadIdx.x & 31;
+    uint4 mask[4] = {}, next[4] = {};
+    auto load_mask = [&](int c) {
+        if constexpr (EPI == EPI_DRELU_BF16) {
+            const uint4* mp = reinterpret_cast<const uint4*>(
+                ep.mask + (size_t)(row0 + lane) * ep.ldm + n0 + c * 32);
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-            o[q] = make_float4(v[4 * q] * s, v[4 * q + 1] * s, v[4 * q + 2] * s,
-                               v[4 * q + 3] * s);
-    } else {
-        uint4* o = reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(ep.out) +
-                                            (size_t)row * ep.ldo + col0);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            uint4 u;
-            u.x = pack_bf16x2(v[8 * q], v[8 * q + 1]);
-            u.y = pack_bf16x2(v[8 * q + 2], v[8 * q + 3]);
-            u.z = pack_bf16x2(v[8 * q + 4], v[8 * q + 5]);
-            u.w = pack_bf16x2(v[8 * q + 6], v[8 * q + 7]);
-            o[q] = u;
+            for (int k = 0; k < 4; ++k) next[k] = mp[k];
         }
-        if (ep.outT) {
-            // Lanes hold consecutive rows: each store writes 64 contiguous
-            // bytes of one transposed row.
-            bf16* t = reinterpret_cast<bf16*>(ep.outT) + (size_t)col0 * ep.ldt + row;
+    };
+    load_mask(part);
+#pragma unroll 1
+    for (int c = part; c < kChunks; c += kPerQ) {
+        uint32_t v[32];
+        tmem_ld32(trow + (uint32_t)(c * 32), v);
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-                t[(size_t)j * ep.ldt] = __float2bfloat16_rn(v[j]);
+        for (int k = 0; k < 4; ++k) mask[k] = next[k];
+        if (c + kPerQ < kChunks) load_mask(c + kPerQ);
+        tmem_wait_ld();
+        if (c + kPerQ >= kChunks) {  // this warp's last chunk: hand it back
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) last();
         }
+        epilogue_chunk<EPI>(v, mask, row0, n0 + c * 32,
+                            ep.bias ? ep.bias + n0 + c * 32 : nullptr, ep, stage);
     }
 }
 
@@ -178,15 +241,16 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[32], int row,
 // and gives up early once another role has failed; the producer then waits
 // for its own loads in flight and the MMA thread for its MMAs before the
 // TMEM is freed.
+constexpr int kEpiWarps = 8;  // two per TMEM lane quarter
 template <int BN>
 struct PTile {
     static constexpr int kStages = BN == 256 ? 4 : 6;
     static constexpr int kABytes = BM * BK * 2;
     static constexpr int kBBytes = BN * BK * 2;
     static constexpr int kRing = kStages * (kABytes + kBBytes);
-    static constexpr int kSmem = kRing + 1024 + 256;  // + alignment, barriers
+    // + the epilogue's stages, alignment, barriers
+    static constexpr int kSmem = kRing + kEpiWarps * kStagedBytes + 1024 + 256;
 };
-constexpr int kEpiWarps = 8;  // two per TMEM lane quarter
 constexpr int kPThreads = 64 + 32 * kEpiWarps;
 
 struct TileGrid {
@@ -209,7 +273,8 @@ __global__ void __launch_bounds__(kPThreads, 1)
     unsigned char* base = smem_raw + ((1024u - (s0 & 1023u)) & 1023u);
     unsigned char* sA = base;
     unsigned char* sB = base + S * kABytes;
-    uint64_t* full = reinterpret_cast<uint64_t*>(base + PTile<BN>::kRing);
+    unsigned char* staged = base + PTile<BN>::kRing;
+    uint64_t* full = reinterpret_cast<uint64_t*>(staged + kEpiWarps * kStagedBytes);
     uint64_t* empty = full + S;
     uint64_t* acc_full = empty + S;   // [2]
     uint64_t* acc_empty = acc_full + 2;  // [2]
@@ -349,21 +414,10 @@ __global__ void __launch_bounds__(kPThreads, 1)
             EpiArgs et = ep;
             if (EPI == EPI_F32)
                 et.out = reinterpret_cast<float*>(ep.out) + (size_t)z * ep.split_stride;
-            const int row = m0 + q * 32 + lane;
             const uint32_t trow = tmem + (uint32_t)(b * BN) + ((uint32_t)(q * 32) << 16);
-#pragma unroll 1
-            for (int c = part; c < kChunks; c += kPerQ) {
-                uint32_t v[32];
-                tmem_ld32(trow + (uint32_t)(c * 32), v);
-                tmem_wait_ld();
-                if (c + kPerQ >= kChunks) {  // this warp's last chunk: hand it back
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&acc_empty[b]);
-                }
-                epilogue_chunk<EPI>(v, row, n0 + c * 32,
-                                    ep.bias ? ep.bias + n0 + c * 32 : nullptr, et);
-            }
+            epilogue_tile<EPI, kChunks, kPerQ>(trow, m0 + q * 32, n0, part, et,
+                                               staged + (warp - 2) * kStagedBytes,
+                                               [&] { mbar_arrive(&acc_empty[b]); });
         }
     }
     tc_fence_before();
@@ -478,8 +532,12 @@ int gemm_bn(cudaStream_t s, MapRef a, MapRef b, int M, int N, int K,
     return 0;
 }
 
-// D = A B^T.  The 128 x 256 tile is used when N allows it and it still gives
-// at least one CTA per SM; otherwise 128 x 128.
+// D = A B^T.  The 128 x 256 tile is used when N allows it and there are more 128 x
+// 128 tiles than SMs: a round of wide tiles takes about one and a half of narrow
+// ones.  Training step with wide and with narrow tiles in the layers this decides:
+// 244 and 256 us at a batch of 4096 (128 or 256 tiles), 308 and 307 at 4864 (152 or
+// 304), 355 and 393 at 8192, 584 and 621 at 16384; 226 and 200 at 2048 (64 or 128,
+// narrow).  Both sum k in the same order: the results are the same bits.
 template <int EPI>
 int gemm(cudaStream_t s, MapRef a, MapRef b, int M, int N, int K,
          const EpiArgs& ep, unsigned* err, int splits = 1) {
@@ -491,7 +549,7 @@ int gemm(cudaStream_t s, MapRef a, MapRef b, int M, int N, int K,
         return -1;
     }
     const bool wide = N % 256 == 0 && b.map->has256 &&
-                      (long long)(M / BM) * (N / 256) * splits >= 148;
+                      (long long)(M / BM) * (N / 128) * splits > sm_count();
     return wide ? gemm_bn<EPI, 256>(s, a, b, M, N, K, ep, err, splits)
                 : gemm_bn<EPI, 128>(s, a, b, M, N, K, ep, err, splits);
 }
