@@ -103,14 +103,37 @@ __host__ __device__ __forceinline__ U4 philox4x32_10(U4 c, uint32_t k0,
     return c;
 }
 
-// Uniform in the open interval (0,1): 23 random bits + 1/2, exact in f32.
+// Uniform in the open interval (0,1): 23 random bits + 1/2, exact in f32.  The
+// device takes the bits as a significand: 1 + m 2^-23, less 1 - 2^-24.
 __host__ __device__ __forceinline__ float u01_open(uint32_t x) {
+#ifdef __CUDA_ARCH__
+    return __fadd_rn(__uint_as_float(0x3F800000u | (x >> 9)), -(1.0f - 0x1p-24f));
+#else
     return ((float)(x >> 9) + 0.5f) * (1.0f / 8388608.0f);
+#endif
 }
 
-// Box-Muller pair (Box & Muller 1958) from two open uniforms.
+// root = RN(sqrt(s)) and, Newton's iteration refined, 1 / root, both from one
+// approximate reciprocal root; the exact residual s - g^2, fused, gives the correctly
+// rounded root (P. Markstein, Computation of elementary functions on the IBM RISC
+// System/6000 processor, IBM J. Res. Dev. 34, 1990).  For s in [2^-58, 2^80], where
+// the residual is exact (equal to sqrtf for every float of that range).
+__device__ __forceinline__ float root_of(float s, float& half_recip) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(s));
+    float g = __fmul_rn(s, y), h = __fmul_rn(0.5f, y);
+    const float e = __fmaf_rn(-h, g, 0.5f);
+    g = __fmaf_rn(g, e, g);
+    h = __fmaf_rn(h, e, h);
+    half_recip = h;
+    return __fmaf_rn(__fmaf_rn(-g, g, s), h, g);
+}
+
+// Box-Muller pair (Box & Muller 1958) from two open uniforms (2^-24 and more below
+// one: the logarithm's root is in root_of's range).
 __device__ __forceinline__ float2 box_muller(float u1, float u2) {
-    float r = sqrtf(-2.0f * logf(u1));
+    float unused;
+    float r = root_of(-2.0f * logf(u1), unused);
     float s, c;
     sincospif(2.0f * u2, &s, &c);
     return make_float2(r * c, r * s);
@@ -202,6 +225,24 @@ __device__ __forceinline__ Quat q_from_axis_angle(float3 axis, float angle) {
     const float h = __fmul_rn(0.5f, angle);
     const float s = __fdiv_rn(sinf(h), nrm);
     return {cosf(h), __fmul_rn(axis.x, s), __fmul_rn(axis.y, s), __fmul_rn(axis.z, s)};
+}
+
+// q_from_axis_angle(axis, |axis|).  In root_of's range the norm and the quotient
+// sin(h) / norm share one reciprocal root (a norm whose significand is all ones, whose
+// reciprocal does not round correctly, excepted), and sin and cos one reduction.
+__device__ __forceinline__ Quat q_from_rotation(float3 v) {
+    const float n2 = __fmaf_rn(v.z, v.z, __fmaf_rn(v.y, v.y, __fmul_rn(v.x, v.x)));
+    float r;
+    const float nrm = root_of(n2, r);
+    if (!(n2 >= 0x1p-58f && n2 <= 0x1p80f) || (~__float_as_uint(nrm) & 0x7FFFFFu) == 0)
+        return q_from_axis_angle(v, norm3(v));
+    r = __fadd_rn(r, r);
+    r = __fmaf_rn(r, __fmaf_rn(-nrm, r, 1.0f), r);
+    float sn, cs;
+    sincosf(__fmul_rn(0.5f, nrm), &sn, &cs);
+    const float q = __fmul_rn(sn, r);
+    const float s = __fmaf_rn(__fmaf_rn(-nrm, q, sn), r, q);
+    return {cs, __fmul_rn(v.x, s), __fmul_rn(v.y, s), __fmul_rn(v.z, s)};
 }
 
 // ------------------------------------------------------------ float keys

@@ -40,7 +40,9 @@ __device__ __forceinline__ void store_pose(const Planes& s, int i, float3 p,
 // Motion model of the reference predict (src/cuda/pf_kernels.cu:198-222,
 // semantics crates/pf_core/src/cpu.rs:197-218): body displacement t + sigma_t*n
 // rotated into the world by q, then q <- (q * q_odo) * exp(sigma_r*w).  The
-// quaternion is not renormalised, as in the reference.
+// quaternion is not renormalised, as in the reference.  Bound by arithmetic: 564
+// issue slots a particle, 200 of them Philox's (652 with the library's roots, the
+// quotient and sin and cos apart).
 __device__ __forceinline__ void apply_predict(const PredictArgs& pa,
                                               uint64_t seed, int i, float3& p,
                                               Quat& q) {
@@ -55,8 +57,7 @@ __device__ __forceinline__ void apply_predict(const PredictArgs& pa,
     p.z += world.z;
     float3 axis = make_float3(pa.rstd[0] * nz[3], pa.rstd[1] * nz[4],
                               pa.rstd[2] * nz[5]);
-    float ang = norm3(axis);
-    Quat dq = q_from_axis_angle(axis, ang);
+    Quat dq = q_from_rotation(axis);
     Quat qo = {pa.q[0], pa.q[1], pa.q[2], pa.q[3]};
     q = q_product(q_product(q, qo), dq);
 }
