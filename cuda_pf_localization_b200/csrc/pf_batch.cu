@@ -192,11 +192,12 @@ __global__ void __launch_bounds__(kWThreads, 6)
     const BTile t = T[blockIdx.x];
     const BFilter& fl = F[t.f];
     BCtl* c = C + t.f;
+    pdl_wait();
     const PfcBatchCycle in = cyc[t.f];
     const Planes s = filter_planes(A, c->live, fl.off);
     PredictArgs pa;
     pa.enabled = 1;
-    pa.gen = c->gen;
+    pa.gen = c->gen + 1ull;  // stored by the filter's last tile
     for (int k = 0; k < 3; ++k) {
         pa.t[k] = in.odom.t[k];
         pa.tstd[k] = in.odom.tstd[k];
@@ -220,7 +221,11 @@ __global__ void __launch_bounds__(kWThreads, 6)
     const int nobs = in.nobs;
     if (nobs <= 0) {
         // predict only: the single-filter cycle resets the weights to uniform
-        if (threadIdx.x == 0 && t.local == 0) c->wmode = WMODE_UNIFORM;
+        if (threadIdx.x == 0 && atomicAdd(&c->done_w, 1u) == (unsigned)fl.nwtiles - 1u) {
+            c->wmode = WMODE_UNIFORM;
+            c->gen = pa.gen;
+            c->done_w = 0u;
+        }
         return;
     }
     float acc0, acc1;
@@ -247,6 +252,7 @@ __global__ void __launch_bounds__(kWThreads, 6)
         const int ok = (ms.y > 0.0f && isfinite(ms.y)) ? 1 : 0;
         c->wvalid = ok;
         c->wmode = ok ? WMODE_LL : WMODE_UNIFORM;
+        c->gen = pa.gen;
         c->done_w = 0u;
     }
 }
@@ -362,6 +368,7 @@ __global__ void __launch_bounds__(kThreads)
     const BTile t = T[blockIdx.x];
     const BFilter& fl = F[t.f];
     BCtl* c = C + t.f;
+    pdl_wait();
     const int wmode = c->wmode;
     const float M = c->M, S = c->S;
     const double rS = __drcp_rn((double)S);
@@ -434,6 +441,7 @@ __global__ void __launch_bounds__(kThreads, 3)
     const BTile t = T[blockIdx.x];
     const BFilter& fl = F[t.f];
     BCtl* c = C + t.f;
+    pdl_wait();
     // a filter that resampled in the last cycle has its sums from k_b_est_src
     if (c->resampled) return;
     const Planes s = filter_planes(A, c->live, fl.off);
@@ -502,6 +510,7 @@ __global__ void __launch_bounds__(kThreads, 3)
     const BTile t = T[blockIdx.x];
     const BFilter& fl = F[t.f];
     BCtl* c = C + t.f;
+    pdl_wait();
     const Planes s = filter_planes(A, c->live, fl.off);
     const int wmode = c->wmode;
     const float M = c->M, S = c->S;
@@ -568,14 +577,18 @@ __global__ void __launch_bounds__(kThreads, 3)
 // filter's tiles are consecutive in that order, so each tile's predecessors
 // are already running when it looks back).  Source j writes j at the first
 // output of its run and at every gather-tile boundary inside it (runs are
-// disjoint, so no two sources write the same marker); k_b_gather copies.
-__global__ void __launch_bounds__(kThreads)
+// disjoint, so no two sources write the same marker); k_b_gather copies.  Its
+// blocks mostly wait (the look-back, FP64 chains): four per SM (64 registers) where
+// 72 registers let three run took a 128-filter cycle of 4.7M particles from 515 to
+// 507 us; five and six were slower.
+__global__ void __launch_bounds__(kThreads, 4)
     k_b_resample(Arena A, const BFilter* __restrict__ F, const BTile* __restrict__ T,
                  BCtl* C, BGlobal* G, unsigned* flags, uint64_t* vals) {
     __shared__ unsigned s_tile;
     __shared__ uint64_t s_warp[kThreads / 32];
     __shared__ uint64_t s_prefix, s_agg;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_wait();
     if (tid == 0) s_tile = atomicAdd(&G->tile_counter, 1u);
     __syncthreads();
     const BTile t = T[s_tile];
@@ -709,6 +722,7 @@ __global__ void __launch_bounds__(kThreads)
     const BTile t = T[blockIdx.x];
     const BFilter& fl = F[t.f];
     const BCtl* c = C + t.f;
+    pdl_wait();
     if (!c->resample_now || !c->resample_valid) return;
     const int n = fl.n;
     int* mk = A.marker + fl.off;
@@ -818,6 +832,7 @@ __global__ void k_b_inject_link(const BFilter* __restrict__ F, const BCtl* C,
     if (d >= total) return;
     const int f = draw_f[d];
     const BCtl& c = C[f];
+    pdl_wait();
     if (!c.resample_now || !c.resample_valid) return;
     const BFilter& fl = F[f];
     const InjDraw dr = inj_draw(c.lcg_next, c.gen, d - fl.inj_off, fl.n);
@@ -840,6 +855,7 @@ __global__ void k_b_inject_apply(Arena A, const BFilter* __restrict__ F,
     if (d >= total) return;
     const int f = draw_f[d];
     const BCtl& c = C[f];
+    pdl_wait();
     if (!c.resample_now || !c.resample_valid) return;
     const BFilter& fl = F[f];
     const uint64_t lcg = c.lcg_next;
@@ -871,40 +887,38 @@ __global__ void k_b_inject_apply(Arena A, const BFilter* __restrict__ F,
     dst.pz[dr.idx] = pz;
 }
 
-__global__ void k_b_commit(BCtl* C, BGlobal* G, int nf) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f < nf) {
-        BCtl& c = C[f];
-        if (c.resample_now) {
-            if (c.resample_valid) {
-                c.live = 1 - c.live;
-                c.resampled = 1;
-                c.lcg = c.lcg_next;
-            }
-            c.wmode = WMODE_UNIFORM;
-        }
-        if (c.err) atomicOr(&G->err, c.err);
-    }
-    if (f == 0) {
-        G->tile_counter = 0u;
-        unsigned e = (G->scan_epoch + 1u) & 0x3FFFFFFFu;
-        G->scan_epoch = e ? e : 1u;
-        e = G->inj_epoch + 1u;
-        G->inj_epoch = e ? e : 1u;
-    }
-}
-
-// Estimate sums of a filter that resampled this cycle, without a pass over
-// the new cloud: its gather tiles' sums in tile order, plus wd times the
+// Commits every filter's resample and readies the batch for the next one; then the
+// estimate sums of a filter that resampled, without a pass over the new cloud: its gather tiles' sums in tile order, plus wd times the
 // injection's position changes in draw order; then the Markley mean and the
 // f32 means of the covariance pass, as the estimate pass's last tile leaves
 // them.  One block per filter; the others take the estimate pass.
 __global__ void __launch_bounds__(kThreads)
-    k_b_est_src(const BFilter* __restrict__ F, BCtl* C, const double* __restrict__ gpart,
-                const double* __restrict__ icorr) {
+    k_b_est_src(const BFilter* __restrict__ F, BCtl* C, BGlobal* G,
+                const double* __restrict__ gpart, const double* __restrict__ icorr) {
     const BFilter& fl = F[blockIdx.x];
     BCtl* c = C + blockIdx.x;
-    if (!c->resampled) return;
+    pdl_wait();
+    const bool resampled = c->resample_now ? c->resample_valid : c->resampled;
+    __syncthreads();  // before the first thread's stores
+    if (threadIdx.x == 0) {
+        if (c->resample_now) {
+            if (c->resample_valid) {
+                c->live = 1 - c->live;
+                c->resampled = 1;
+                c->lcg = c->lcg_next;
+            }
+            c->wmode = WMODE_UNIFORM;
+        }
+        if (c->err) atomicOr(&G->err, c->err);
+        if (blockIdx.x == 0) {
+            G->tile_counter = 0u;
+            unsigned e = (G->scan_epoch + 1u) & 0x3FFFFFFFu;
+            G->scan_epoch = e ? e : 1u;
+            e = G->inj_epoch + 1u;
+            G->inj_epoch = e ? e : 1u;
+        }
+    }
+    if (!resampled) return;
     __shared__ double s_out[kEstN];
     tiles_combine<kEstN>(gpart + (size_t)fl.gtile0 * kEstN, fl.ngtiles, s_out);
     double qm[4];
@@ -1079,43 +1093,40 @@ int rebuild_est_tiles(BatchHandle* h) {
 }
 
 int launch_est_covs(BatchHandle* h) {
-    k_b_est<<<h->n_et, kThreads, 0, h->stream>>>(h->A, h->d_F, h->d_et, h->d_C,
-                                                 h->d_epart);
-    k_b_covs<<<h->n_et, kThreads, 0, h->stream>>>(h->A, h->d_F, h->d_et, h->d_C,
-                                                  h->d_cpart, h->d_out);
+    PFB_CK(launch_pdl(k_b_est, h->n_et, kThreads, 0, h->stream, h->A, h->d_F, h->d_et, h->d_C,
+                      h->d_epart));
+    PFB_CK(launch_pdl(k_b_covs, h->n_et, kThreads, 0, h->stream, h->A, h->d_F, h->d_et, h->d_C,
+                      h->d_cpart, h->d_out));
     h->launches += 2;
     PFB_KL();
     return 0;
 }
 
-// The kernel chain of one cycle on h->stream (inputs in d_cyc / d_obs).
+// The kernel chain of one cycle on h->stream (inputs in d_cyc / d_obs), each kernel
+// launched while the one before drains.
 int enqueue_cycle(BatchHandle* h) {
     cudaStream_t s = h->stream;
-    k_b_gen_inc<<<ceil_div(h->nf, kThreads), kThreads, 0, s>>>(h->d_C, h->nf);
-    k_b_weight<<<h->n_wt, kWThreads, 0, s>>>(h->A, h->d_F, h->d_wt, h->d_C, h->d_cyc,
-                                            h->d_obs, h->d_lm, h->d_wpart,
-                                            h->use_packed);
-    k_b_ess<<<h->n_et, kThreads, 0, s>>>(h->A, h->d_F, h->d_et, h->d_C, h->d_epart,
-                                         h->d_eupart, h->d_out);
-    h->launches += 3;
-    PFB_KL();
-    k_b_resample<<<h->n_rt, kThreads, 0, s>>>(h->A, h->d_F, h->d_rt, h->d_C, h->d_G,
-                                              h->d_flags, h->d_vals);
-    k_b_gather<<<h->n_gt, kThreads, 0, s>>>(h->A, h->d_F, h->d_gt, h->d_C, h->d_gpart);
-    h->launches += 2;
+    PFB_CK(launch_pdl(k_b_weight, h->n_wt, kWThreads, 0, s, h->A, h->d_F, h->d_wt, h->d_C,
+                      h->d_cyc, h->d_obs, h->d_lm, h->d_wpart, h->use_packed));
+    PFB_CK(launch_pdl(k_b_ess, h->n_et, kThreads, 0, s, h->A, h->d_F, h->d_et, h->d_C,
+                      h->d_epart, h->d_eupart, h->d_out));
+    PFB_CK(launch_pdl(k_b_resample, h->n_rt, kThreads, 0, s, h->A, h->d_F, h->d_rt, h->d_C,
+                      h->d_G, h->d_flags, h->d_vals));
+    PFB_CK(launch_pdl(k_b_gather, h->n_gt, kThreads, 0, s, h->A, h->d_F, h->d_gt, h->d_C,
+                      h->d_gpart));
+    h->launches += 4;
     if (h->total_draws > 0) {
         const int g = ceil_div(h->total_draws, kThreads);
-        k_b_inject_link<<<g, kThreads, 0, s>>>(h->d_F, h->d_C, h->d_G, h->d_draw_f,
-                                               h->total_draws, h->d_inj_head,
-                                               h->d_inj_next);
-        k_b_inject_apply<<<g, kThreads, 0, s>>>(h->A, h->d_F, h->d_C, h->d_G,
-                                                h->d_draw_f, h->total_draws,
-                                                h->d_inj_head, h->d_inj_next, h->d_icorr);
+        PFB_CK(launch_pdl(k_b_inject_link, g, kThreads, 0, s, h->d_F, h->d_C, h->d_G,
+                          h->d_draw_f, h->total_draws, h->d_inj_head, h->d_inj_next));
+        PFB_CK(launch_pdl(k_b_inject_apply, g, kThreads, 0, s, h->A, h->d_F, h->d_C, h->d_G,
+                          h->d_draw_f, h->total_draws, h->d_inj_head, h->d_inj_next,
+                          h->d_icorr));
         h->launches += 2;
     }
-    k_b_commit<<<ceil_div(h->nf, kThreads), kThreads, 0, s>>>(h->d_C, h->d_G, h->nf);
-    k_b_est_src<<<h->nf, kThreads, 0, s>>>(h->d_F, h->d_C, h->d_gpart, h->d_icorr);
-    h->launches += 2;
+    PFB_CK(launch_pdl(k_b_est_src, h->nf, kThreads, 0, s, h->d_F, h->d_C, h->d_G, h->d_gpart,
+                      h->d_icorr));
+    h->launches += 1;
     PFB_KL();
     if (launch_est_covs(h)) return -1;
     PFB_CK(cudaMemcpyAsync(h->h_G, h->d_G, sizeof(BGlobal), cudaMemcpyDeviceToHost, s));
