@@ -162,35 +162,49 @@ static __device__ __noinline__ void markley_mean_serial(const double* m10, doubl
     markley_mean(m10, q_out);
 }
 
+// A power of two that brings x > 0 (normal, finite) into [1, 2).
+__device__ __forceinline__ double exponent_scale(double x) {
+    return __hiloint2double((2046 - ((__double2hiint(x) >> 20) & 0x7FF)) << 20, 0);
+}
+
 // markley_mean by one warp: lanes 4r + c (r, c < 4) of the first 16 hold
 // element (r, c) of the 4x4 matrix, so a squaring is four shuffled products
 // per lane instead of 64 serial ones; the same method and acceptance test as
 // dominant_eigvec_psd4, and the same serial Jacobi fallback (one lane) for a
-// near-degenerate top eigenvalue.  Every lane of the warp must call it; the
-// result is valid in every lane.
+// near-degenerate top eigenvalue.  It is a serial chain that a whole grid may wait
+// for, so the squarings are scaled by powers of two and the power steps not at all:
+// one root and one quotient in all, at the end (in place of a quotient a squaring
+// and two roots and quotients in the steps and the test: FIGM).  Every lane of the
+// warp must call it; the result is valid in every lane.
 __device__ inline void markley_mean_warp(const double m10[10], double q_out[4]) {
     const unsigned full = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31;
     const int r = (lane >> 2) & 3, c = lane & 3;
     const int lo = r < c ? r : c, hi = r < c ? c : r;
-    const double a = m10[lo * 4 - lo * (lo - 1) / 2 + (hi - lo)];  // a[r][c]
+    double a = m10[lo * 4 - lo * (lo - 1) / 2 + (hi - lo)];  // a[r][c]
     auto at = [&](double v, int rr, int cc) { return __shfl_sync(full, v, rr * 4 + cc); };
     auto trace = [&](double v) {
-        return at(v, 0, 0) + at(v, 1, 1) + at(v, 2, 2) + at(v, 3, 3);
+        return (at(v, 0, 0) + at(v, 1, 1)) + (at(v, 2, 2) + at(v, 3, 3));
     };
-    const double tr = trace(a);
-    bool ok = tr > 0.0;
+    double tr = trace(a);
+    bool ok = tr >= 1e-290 && tr <= 1e290;
     double x[4] = {0.0, 0.0, 0.0, 0.0};
+    double xx = 0.0;
     if (ok) {
-        const double itr = 1.0 / tr;
-        double pm = a * itr;
+        const double s0 = exponent_scale(tr);
+        a *= s0;
+        tr *= s0;
+        double pm = a, tp = tr;  // a scaled power of a and its trace, in [1, 2)
         for (int s = 0; s < 12 && ok; ++s) {
-            const double t = at(pm, r, 0) * at(pm, 0, c) + at(pm, r, 1) * at(pm, 1, c) +
-                             at(pm, r, 2) * at(pm, 2, c) + at(pm, r, 3) * at(pm, 3, c);
+            const double t = fma(at(pm, r, 0), at(pm, 0, c), at(pm, r, 1) * at(pm, 1, c)) +
+                             fma(at(pm, r, 2), at(pm, 2, c), at(pm, r, 3) * at(pm, 3, c));
             const double tt = trace(t);
             ok = tt > 0.0;
-            pm = t * (1.0 / tt);
-            if (tt > 1.0 - 1e-14) break;  // warp-uniform: every lane has tt
+            const double sc = exponent_scale(tt);
+            const bool rank_one = tt > (1.0 - 1e-14) * (tp * tp);
+            pm = t * sc;
+            tp = tt * sc;
+            if (rank_one) break;  // warp-uniform: every lane has tt
         }
         if (ok) {
             // the column of the largest diagonal entry, then two power steps
@@ -204,43 +218,43 @@ __device__ inline void markley_mean_warp(const double m10[10], double q_out[4]) 
                     cb = i;
                 }
             }
+            double am[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) am[i] = __shfl_sync(full, a, i);
             for (int i = 0; i < 4; ++i) x[i] = at(pm, i, cb);
-            for (int it = 0; it < 2 && ok; ++it) {
-                double y[4];
+            double y[4];
+            auto step = [&]() {
+#pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    y[i] = at(a, i, 0) * x[0] + at(a, i, 1) * x[1] + at(a, i, 2) * x[2] +
-                           at(a, i, 3) * x[3];
-                const double ny = sqrt(y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3]);
-                ok = ny > 0.0;
-                for (int i = 0; i < 4; ++i) x[i] = y[i] / ny;
+                    y[i] = fma(am[4 * i], x[0], am[4 * i + 1] * x[1]) +
+                           fma(am[4 * i + 2], x[2], am[4 * i + 3] * x[3]);
+            };
+            for (int it = 0; it < 2; ++it) {
+                step();
+                for (int i = 0; i < 4; ++i) x[i] = y[i];
             }
-            if (ok) {
-                double y[4];
-                for (int i = 0; i < 4; ++i)
-                    y[i] = at(a, i, 0) * x[0] + at(a, i, 1) * x[1] + at(a, i, 2) * x[2] +
-                           at(a, i, 3) * x[3];
-                const double lam = x[0] * y[0] + x[1] * y[1] + x[2] * y[2] + x[3] * y[3];
-                double res = 0.0;
-                for (int i = 0; i < 4; ++i) res += (y[i] - lam * x[i]) * (y[i] - lam * x[i]);
-                ok = sqrt(res) <= 1e-13 * tr;
+            step();
+            xx = fma(x[0], x[0], x[1] * x[1]) + fma(x[2], x[2], x[3] * x[3]);
+            const double xy = fma(x[0], y[0], x[1] * y[1]) + fma(x[2], y[2], x[3] * y[3]);
+            // |a v - (v' a v) v|^2 for v = x / |x|, times |x|^6
+            double res = 0.0;
+            for (int i = 0; i < 4; ++i) {
+                const double d = xx * y[i] - xy * x[i];
+                res = fma(d, d, res);
             }
+            ok = xx > 0.0 && res <= 1e-26 * (tr * tr) * (xx * xx * xx);
         }
     }
     if (!ok) {
-        // near-degenerate spectrum: the serial solve, by lane 0
+        // near-degenerate spectrum (or a sum out of range): the serial solve, by lane 0
         double q[4];
         if (lane == 0) markley_mean_serial(m10, q);
         for (int i = 0; i < 4; ++i) q_out[i] = __shfl_sync(full, q[i], 0);
         return;
     }
-    const double nrm = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3]);
-    if (!(nrm > 0.0)) {
-        q_out[0] = 1.0;
-        q_out[1] = q_out[2] = q_out[3] = 0.0;
-        return;
-    }
-    const double sgn = (x[0] < 0.0) ? -1.0 : 1.0;
-    for (int i = 0; i < 4; ++i) q_out[i] = sgn * x[i] / nrm;
+    const double own = c == 0 ? x[0] : c == 1 ? x[1] : c == 2 ? x[2] : x[3];
+    const double q = (x[0] < 0.0 ? -own : own) / sqrt(xx);
+    for (int i = 0; i < 4; ++i) q_out[i] = __shfl_sync(full, q, i);
 }
 
 // markley_mean_warp as a call of its own: not inlined, so its registers do

@@ -257,23 +257,18 @@ __global__ void __launch_bounds__(kWThreads, 6)
     }
 }
 
-// Block partial of NV FP64 sums (fixed order) into part[NV]; returns true in
-// every thread of the filter's last tile after its partials are visible.
-// Block partial of NV per-thread FP64 accumulators (xor butterfly per warp,
-// warps in order) into part[0..NV).
+// Block partial of NV per-thread FP64 accumulators (a butterfly per warp, warps in
+// order; acc is used up) into part[0..NV).
 template <int NV>
 __device__ __forceinline__ void block_partial(double (&acc)[NV], double* part) {
-    __shared__ double s_w[NV][kThreads / 32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        const double v = warp_sum_d(acc[k]);
-        if (lane == 0) s_w[k][warp] = v;
-    }
+    __shared__ double s_w[kThreads / 32][NV];
+    const int tid = threadIdx.x;
+    const int q = warp_sums(acc);
+    if (q >= 0) s_w[tid >> 5][q] = acc[0];
     __syncthreads();
     if (tid < NV) {
         double v = 0.0;
-        for (int k = 0; k < kThreads / 32; ++k) v += s_w[tid][k];
+        for (int k = 0; k < kThreads / 32; ++k) v += s_w[k][tid];
         part[tid] = v;
     }
 }
@@ -285,22 +280,21 @@ __device__ __forceinline__ bool tile_partial(double (&acc)[NV], double* part,
                                              unsigned* done, int ntiles) {
     __shared__ bool s_last;
     block_partial<NV>(acc, part);
-    __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) s_last = (atomicAdd(done, 1u) == (unsigned)ntiles - 1u);
+    if (threadIdx.x == 0) s_last = atomic_add_acq_rel(done, 1u) == (unsigned)ntiles - 1u;
     __syncthreads();
-    if (!s_last) return false;
-    __threadfence();
-    return true;
+    return s_last;
 }
 
-// Sum of the filter's tile partials in tile order (warp k: component k).
+// Sum of the filter's tile partials in tile order (warp k: component k), loads
+// ahead of the sums.
 template <int NV>
 __device__ __forceinline__ void tiles_combine(const double* part, int ntiles,
                                               double* out) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int k = warp; k < NV; k += kThreads / 32) {
         double v = 0.0;
+#pragma unroll 4
         for (int b = lane; b < ntiles; b += 32) v += __ldcg(&part[(size_t)b * NV + k]);
         v = warp_sum_d(v);
         if (lane == 0) out[k] = v;
@@ -925,6 +919,7 @@ __global__ void __launch_bounds__(kThreads)
     if (threadIdx.x < 32) {
         const int lane = threadIdx.x;
         double d[3] = {0.0, 0.0, 0.0};
+#pragma unroll 8
         for (int j = lane; j < fl.inj_k; j += 32)
 #pragma unroll
             for (int q = 0; q < 3; ++q) d[q] += icorr[3 * (size_t)(fl.inj_off + j) + q];

@@ -165,6 +165,102 @@ __device__ __forceinline__ double warp_sum_d(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(~0u, v, o);
     return v;
 }
+// warp_sum_d of NV <= 16 values at once, the values divided among the lanes as the
+// butterfly goes: 26 shuffled words for NV = 14 where one at a time takes 140.  Every
+// sum is formed in warp_sum_d's order.  Leaves a lane's sum in v[0] and returns which
+// value it is of, or -1.
+template <int N, int O, int NV>
+__device__ __forceinline__ int warp_sums_from(double (&v)[NV]) {
+    const bool up = threadIdx.x & O;
+    if constexpr (O == 0) {
+        return 0;
+    } else if constexpr (N == 1) {
+        v[0] += __shfl_xor_sync(~0u, v[0], O);
+        const int q = warp_sums_from<1, O / 2>(v);
+        return up ? -1 : q;
+    } else {
+        constexpr int H = (N + 1) / 2;  // the lanes with the bit set keep the upper ones
+#pragma unroll
+        for (int i = 0; i < H; ++i) {
+            const double lo = v[i], hi = i + H < N ? v[i + H < N ? i + H : 0] : 0.0;
+            v[i] = (up ? hi : lo) + __shfl_xor_sync(~0u, up ? lo : hi, O);
+        }
+        const int q = warp_sums_from<H, O / 2>(v);
+        return q < 0 ? -1 : !up ? q : q + H < N ? q + H : -1;
+    }
+}
+template <int NV>
+__device__ __forceinline__ int warp_sums(double (&v)[NV]) {
+    static_assert(NV <= 16, "one value a lane after four halvings");
+    return warp_sums_from<NV, 16>(v);
+}
+
+__device__ __forceinline__ unsigned atomic_add_acq_rel(unsigned* p, unsigned v) {
+    unsigned old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
+                 : "=r"(old)
+                 : "l"(p), "r"(v)
+                 : "memory");
+    return old;
+}
+
+// Block sums of NV per-thread FP64 values (acc is used up): a butterfly per warp, the
+// warps in order, value q to part[q * stride + blockIdx.x].
+template <int NV, int kWarps>
+__device__ __forceinline__ void block_partials(double (&acc)[NV], double* part, int stride) {
+    __shared__ double s_w[kWarps][NV];
+    const int q = warp_sums(acc);
+    if (q >= 0) s_w[threadIdx.x >> 5][q] = acc[0];
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        double v = 0.0;
+        for (int k = 0; k < kWarps; ++k) v += s_w[k][threadIdx.x];
+        part[(size_t)threadIdx.x * stride + blockIdx.x] = v;
+    }
+}
+
+// block_partials, then whether this block is the grid's last to get here (the others'
+// partials are visible to all its threads).
+template <int NV, int kWarps>
+__device__ __forceinline__ bool block_partials_last(double (&acc)[NV], double* part, int stride,
+                                                    unsigned* done) {
+    __shared__ bool s_last;
+    block_partials<NV, kWarps>(acc, part, stride);
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomic_add_acq_rel(done, 1u) == gridDim.x - 1;
+    __syncthreads();
+    return s_last;
+}
+
+// The sums of G <= kMaxG blocks' partials (part[q * kMaxG + b]) into s_out[0, NV), by
+// one block: a warp per value, the blocks strided over its lanes, then a butterfly.
+// All of a warp's loads are in flight at once.
+template <int NV, int kMaxG, int kWarps>
+__device__ __forceinline__ void combine_partials(const double* part, int G, double* s_out) {
+    constexpr int kRounds = (NV + kWarps - 1) / kWarps, kPer = (kMaxG + 31) / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double v[kRounds][kPer];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+        const int q = warp + r * kWarps;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+            const int b = lane + 32 * i;
+            v[r][i] = q < NV && b < G ? __ldcg(&part[(size_t)q * kMaxG + b]) : 0.0;
+        }
+    }
+    double a[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+        a[r] = 0.0;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) a[r] += v[r][i];
+    }
+    const int r = warp_sums(a);
+    if (r >= 0 && warp + r * kWarps < NV) s_out[warp + r * kWarps] = a[0];
+    __syncthreads();
+}
+
 __device__ __forceinline__ double warp_max_d(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(~0u, v, o));
@@ -424,9 +520,22 @@ __device__ __forceinline__ float2 softmax_combine(const float2* part, int G) {
     __shared__ float s_r;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid >= kWThreads) G = 0;
+    // a small grid's partials are read once
+    constexpr int kKeep = 4;
+    const bool keep = G <= kKeep * kWThreads;
+    float2 kept[kKeep];
     float mx = -INFINITY;
+    if (keep) {
+#pragma unroll
+        for (int r = 0; r < kKeep; ++r) {
+            const int b = tid + r * kWThreads;
+            kept[r] = b < G ? __ldcg(&part[b]) : make_float2(-INFINITY, 0.0f);
+            mx = fmaxf(mx, kept[r].x);
+        }
+    } else {
 #pragma unroll 4
-    for (int b = tid; b < G; b += kWThreads) mx = fmaxf(mx, __ldcg(&part[b].x));
+        for (int b = tid; b < G; b += kWThreads) mx = fmaxf(mx, __ldcg(&part[b].x));
+    }
     mx = warp_max_f(mx);
     if (lane == 0 && tid < kWThreads) s_d[warp] = mx;
     __syncthreads();
@@ -438,10 +547,16 @@ __device__ __forceinline__ float2 softmax_combine(const float2* part, int G) {
     __syncthreads();
     const float M = s_r;
     float sum = 0.0f;
-#pragma unroll 4
-    for (int b = tid; b < G; b += kWThreads) {
-        const float2 pb = __ldcg(&part[b]);
+    auto add = [&](float2 pb) {
         sum = __fadd_rn(sum, __fmul_rn(expf(__fsub_rn(pb.x, M)), pb.y));
+    };
+    if (keep) {
+#pragma unroll
+        for (int r = 0; r < kKeep; ++r)
+            if (tid + r * kWThreads < G) add(kept[r]);
+    } else {
+#pragma unroll 4
+        for (int b = tid; b < G; b += kWThreads) add(__ldcg(&part[b]));
     }
     sum = warp_sum_f(sum);
     __syncthreads();

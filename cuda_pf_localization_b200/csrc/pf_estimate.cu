@@ -39,58 +39,16 @@ constexpr int kMaxBlocks = 2 * 148;
 
 PlaneSet plane_set(const PfHandle* h) { return {h->planes(0), h->planes(1)}; }
 
-// Reduce NV per-thread FP64 accumulators over the block into part[blk*NV+k];
-// the last block to finish sums the partials of all blocks (G <= kMaxBlocks)
-// in block order into out[k] and returns true (in every thread of that
-// block).  The last block first stages every partial in shared memory with
-// one round of loads, so the combine costs one L2 round trip.
+// Sums of NV per-thread FP64 accumulators over the grid (at most kMaxBlocks blocks)
+// by its last block, in block order, into out[k]; returns true in every thread of
+// that block.
 template <int NV>
 __device__ bool block_reduce_last(double (&acc)[NV], double* part,
                                   unsigned* done, double* out) {
-    __shared__ double s_w[NV][kThreads / 32];
-    __shared__ double s_p[NV * kMaxBlocks];  // [k][block]
-    __shared__ bool s_last;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        double v = warp_sum_d(acc[k]);
-        if (lane == 0) s_w[k][warp] = v;
-    }
-    __syncthreads();
-    if (tid < NV) {
-        double v = 0.0;
-        for (int k = 0; k < kThreads / 32; ++k) v += s_w[tid][k];
-        part[(size_t)blockIdx.x * NV + tid] = v;
-        __threadfence();
-    }
-    __syncthreads();
-    if (tid == 0) s_last = (atomicAdd(done, 1u) == gridDim.x - 1);
-    __syncthreads();
-    if (!s_last) return false;
-    __threadfence();
-    const int G = gridDim.x;
-    const int tot = G * NV;
-    constexpr int kPer = (NV * kMaxBlocks + kThreads - 1) / kThreads;
-    double v[kPer];
-#pragma unroll
-    for (int r = 0; r < kPer; ++r) {
-        const int idx = tid + r * kThreads;
-        v[r] = idx < tot ? __ldcg(&part[idx]) : 0.0;
-    }
-#pragma unroll
-    for (int r = 0; r < kPer; ++r) {
-        const int idx = tid + r * kThreads;
-        if (idx < tot) s_p[(idx % NV) * kMaxBlocks + idx / NV] = v[r];
-    }
-    __syncthreads();
-    for (int k = warp; k < NV; k += kThreads / 32) {
-        double a = 0.0;
-        for (int b = lane; b < G; b += 32) a += s_p[k * kMaxBlocks + b];
-        a = warp_sum_d(a);
-        if (lane == 0) out[k] = a;
-    }
-    __syncthreads();
-    if (tid == 0) *done = 0u;
+    constexpr int kWarps = kThreads / 32;
+    if (!block_partials_last<NV, kWarps>(acc, part, kMaxBlocks, done)) return false;
+    combine_partials<NV, kMaxBlocks, kWarps>(part, gridDim.x, out);
+    if (threadIdx.x == 0) *done = 0u;
     return true;
 }
 
@@ -276,11 +234,19 @@ __global__ void __launch_bounds__(kThreads)
           unsigned* done, CycleCtl* ctl, int decide, double ess_ratio) {
     pdl_wait();
     static_assert(kPrefixBlock == 8 * kThreads, "two float4 per thread");
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // the log-likelihoods go out together with the control block's loads
+    float4 L[2];
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+        const int i4 = blockIdx.x * 2 * kThreads + hh * kThreads + tid;
+        L[hh] = 4 * i4 < n ? reinterpret_cast<const float4*>(ll)[i4]
+                           : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     const int wmode = ctl->wmode;
     const float M = ctl->ll_max, S = ctl->ll_sumexp;
     const double rS = __drcp_rn((double)S);
     const float wuni = 1.0f / (float)n;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double sq = 0.0;
     unsigned long long tfx = 0;
     int bad = 0;
@@ -294,9 +260,8 @@ __global__ void __launch_bounds__(kThreads)
         } else if (wmode == WMODE_UNIFORM) {
             W = make_float4(wuni, wuni, wuni, wuni);
         } else {
-            const float4 L = reinterpret_cast<const float4*>(ll)[i4];
-            W = make_float4(weight_from_ll(L.x, M, S, rS), weight_from_ll(L.y, M, S, rS),
-                            weight_from_ll(L.z, M, S, rS), weight_from_ll(L.w, M, S, rS));
+            W = make_float4(weight_from_ll(L[hh].x, M, S, rS), weight_from_ll(L[hh].y, M, S, rS),
+                            weight_from_ll(L[hh].z, M, S, rS), weight_from_ll(L[hh].w, M, S, rS));
             reinterpret_cast<float4*>(w)[i4] = W;
         }
 #pragma unroll
@@ -331,35 +296,43 @@ __global__ void __launch_bounds__(kThreads)
         part[blockIdx.x] = a;
         partu[2 * (size_t)blockIdx.x] = u;
         partu[2 * (size_t)blockIdx.x + 1] = any_bad ? 1ull : 0ull;
-        __threadfence();
-        s_last = (atomicAdd(done, 1u) == gridDim.x - 1);
+        s_last = atomic_add_acq_rel(done, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!s_last) return;
-    __threadfence();
     // Last block: sum w^2 over the block partials, and the exclusive prefix
-    // of the block totals (each thread scans a contiguous range of blocks).
-    // Up to kStage block totals are staged in shared memory with all loads
-    // in flight at once; larger grids read them from L2 twice.
+    // of the block totals (each thread scans a contiguous range of blocks; up to
+    // kThreads blocks, one each).  Larger grids, up to kStage blocks, stage the
+    // totals in shared memory with all loads in flight at once; the largest read
+    // them from L2 twice.
     const int G = gridDim.x;
     double a = 0.0;
     int fb = 0;
-#pragma unroll 4
-    for (int b = tid; b < G; b += kThreads) {
-        a += __ldcg(&part[b]);
-        fb |= __ldcg(&partu[2 * (size_t)b + 1]) != 0ull ? 1 : 0;
-    }
-    a = warp_sum_d(a);
-    const bool staged = G <= kStage;
-    if (staged) {
-#pragma unroll 4
-        for (int b = tid; b < G; b += kThreads) s_tot[b] = __ldcg(&partu[2 * (size_t)b]);
-    }
-    __syncthreads();
+    unsigned long long run = 0;
+    const bool one = G <= kThreads, staged = !one && G <= kStage;
     const int per = (G + kThreads - 1) / kThreads;
     const int b0 = min(G, tid * per), b1 = min(G, b0 + per);
-    unsigned long long run = 0;
-    for (int b = b0; b < b1; ++b) run += staged ? s_tot[b] : __ldcg(&partu[2 * (size_t)b]);
+    if (one) {
+        if (tid < G) {
+            a += __ldcg(&part[tid]);
+            run = __ldcg(&partu[2 * (size_t)tid]);
+            fb = __ldcg(&partu[2 * (size_t)tid + 1]) != 0ull ? 1 : 0;
+        }
+        a = warp_sum_d(a);
+    } else {
+#pragma unroll 4
+        for (int b = tid; b < G; b += kThreads) {
+            a += __ldcg(&part[b]);
+            fb |= __ldcg(&partu[2 * (size_t)b + 1]) != 0ull ? 1 : 0;
+        }
+        a = warp_sum_d(a);
+        if (staged) {
+#pragma unroll 4
+            for (int b = tid; b < G; b += kThreads) s_tot[b] = __ldcg(&partu[2 * (size_t)b]);
+        }
+        __syncthreads();
+        for (int b = b0; b < b1; ++b) run += staged ? s_tot[b] : __ldcg(&partu[2 * (size_t)b]);
+    }
     // block-exclusive scan of the thread ranges
     unsigned long long x = run;
 #pragma unroll
@@ -376,9 +349,13 @@ __global__ void __launch_bounds__(kThreads)
         T += s_u[k];
     }
     unsigned long long off = wbase + x - run;
-    for (int b = b0; b < b1; ++b) {
-        prefix[b] = off;
-        off += staged ? s_tot[b] : __ldcg(&partu[2 * (size_t)b]);
+    if (one) {
+        if (tid < G) prefix[tid] = off;
+    } else {
+        for (int b = b0; b < b1; ++b) {
+            prefix[b] = off;
+            off += staged ? s_tot[b] : __ldcg(&partu[2 * (size_t)b]);
+        }
     }
     if (tid == 0) {
         double sum = 0.0;

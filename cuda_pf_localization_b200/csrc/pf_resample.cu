@@ -109,76 +109,40 @@ __device__ __forceinline__ Offsets offsets(const CycleCtl* ctl, int n, int use_u
     return o;
 }
 
-// Block sum of NV per-thread FP64 values (xor butterfly per warp, warps in
-// order) into part[blockIdx.x * NV + q]; then whether this block was the last
-// of the grid to finish (counter `done`).  Valid in every thread.
-template <int NV>
-__device__ __forceinline__ bool block_partial_last(const double (&acc)[NV], double* part,
-                                                   unsigned* done) {
-    __shared__ double s_w[NV][kThreads / 32];
-    __shared__ bool s_last;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-        const double x = warp_sum_d(acc[q]);
-        if (lane == 0) s_w[q][warp] = x;
-    }
-    __syncthreads();
-    if (tid < NV) {
-        double x = 0.0;
-        for (int k = 0; k < kThreads / 32; ++k) x += s_w[tid][k];
-        part[(size_t)blockIdx.x * NV + tid] = x;
-        __threadfence();
-    }
-    __syncthreads();
-    if (tid == 0) s_last = atomicAdd(done, 1u) == gridDim.x - 1;
-    __syncthreads();
-    return s_last;
-}
-
-// The last block's combine: the G <= kMaxG partials of NV sums
-// (part[b * NV + q]) staged in shared memory with one round of loads, then
-// summed per component in block order (lanes strided, then a butterfly).
-// Results in s_out[0, NV).
-template <int NV, int kMaxG>
-__device__ __forceinline__ void combine_staged(const double* part, int G, double* s_p,
-                                               double* s_out) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int tot = G * NV;
-    constexpr int kPer = (NV * kMaxG + kThreads - 1) / kThreads;
-    constexpr int kBatch = 8;  // loads in flight per thread
-#pragma unroll 1
-    for (int r0 = 0; r0 < kPer; r0 += kBatch) {
-        double v[kBatch];
-#pragma unroll
-        for (int r = 0; r < kBatch; ++r) {
-            const int idx = tid + (r0 + r) * kThreads;
-            v[r] = idx < tot ? __ldcg(&part[idx]) : 0.0;
-        }
-#pragma unroll
-        for (int r = 0; r < kBatch; ++r) {
-            const int idx = tid + (r0 + r) * kThreads;
-            if (idx < tot) s_p[(idx % NV) * kMaxG + idx / NV] = v[r];
-        }
-    }
-    __syncthreads();
-    for (int q = warp; q < NV; q += kThreads / 32) {
-        double x = 0.0;
-        for (int b = lane; b < G; b += 32) x += s_p[q * kMaxG + b];
-        x = warp_sum_d(x);
-        if (lane == 0) s_out[q] = x;
-    }
-    __syncthreads();
-}
-
 // Injection draws of one tile, in shared memory: local output, draw index,
-// jitter.
+// jitter, the next listed draw on the same output.
 struct InjList {
     int loc[kThreads];
     int j[kThreads];
     float jx[kThreads], jy[kThreads], jz[kThreads];
-    unsigned hit[kTile / 32];  // outputs of the tile hit by a listed draw
+    int next[kThreads];
 };
+
+// One listed draw on a value triple; the exact change (differences of two f32
+// values) goes to d[0..2].
+__device__ __forceinline__ void apply_draw(const InjList& L, int e, float& x, float& y, float& z,
+                                           double (&d)[kCorrN]) {
+    const float nx = x + L.jx[e], ny = y + L.jy[e], nz = z + L.jz[e];
+    d[0] += (double)nx - (double)x;
+    d[1] += (double)ny - (double)y;
+    d[2] += (double)nz - (double)z;
+    x = nx;
+    y = ny;
+    z = nz;
+}
+
+// Apply the draws chained from `head` to one output, in ascending draw order.
+__device__ __forceinline__ void apply_chain(const InjList& L, int head, float& x, float& y,
+                                            float& z, double (&d)[kCorrN]) {
+    for (int last = -1;;) {
+        int best = -1;
+        for (int e = head; e >= 0; e = L.next[e])
+            if (L.j[e] > last && (best < 0 || L.j[e] < L.j[best])) best = e;
+        if (best < 0) break;
+        apply_draw(L, best, x, y, z, d);
+        last = L.j[best];
+    }
+}
 
 // Apply to the group of outputs [l0, l0 + kGroup), in ascending draw order,
 // the listed draws (m entries, any order) that hit it; the exact change of
@@ -198,17 +162,7 @@ __device__ __forceinline__ void apply_draws(const InjList& L, int m, int l0,
         const int r = L.loc[best] - l0;
 #pragma unroll
         for (int q = 0; q < kGroup; ++q)
-            if (q == r) {
-                const float nx = x[q] + L.jx[best], ny = y[q] + L.jy[best],
-                            nz = z[q] + L.jz[best];
-                // exact: differences of two f32 values
-                d[0] += (double)nx - (double)x[q];
-                d[1] += (double)ny - (double)y[q];
-                d[2] += (double)nz - (double)z[q];
-                x[q] = nx;
-                y[q] = ny;
-                z[q] = nz;
-            }
+            if (q == r) apply_draw(L, best, x[q], y[q], z[q], d);
         last = L.j[best];
     }
 }
@@ -239,7 +193,6 @@ __global__ void __launch_bounds__(kThreads, 2)
     const bool resample = !cond || ctl->resample_now;
     const bool valid = resample && ctl->w_total_fx != 0 && !ctl->w_bad;
     __shared__ uint64_t s_warp[kThreads / 32];
-    __shared__ double s_w[kEstN][kThreads / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wmode = ctl->wmode;
     const float M = ctl->ll_max, S = ctl->ll_sumexp;
@@ -375,30 +328,16 @@ __global__ void __launch_bounds__(kThreads, 2)
             }
         }
     }
-    // block partial (xor butterfly per warp, warps in order); block 0 of
-    // k_gather combines them
-#pragma unroll
-    for (int q = 0; q < kEstN; ++q) {
-        const double v = warp_sum_d(acc[q]);
-        if (lane == 0) s_w[q][warp] = v;
-    }
-    __syncthreads();
-    if (tid < kEstN) {
-        double v = 0.0;
-        for (int k = 0; k < kThreads / 32; ++k) v += s_w[tid][k];
-        part_m[(size_t)blockIdx.x * kEstN + tid] = v;
-    }
+    // block 0 of k_gather combines them
+    block_partials<kEstN, kThreads / 32>(acc, part_m, kMarkGrid);
 }
 
-// Shared memory of k_gather: a tile's ancestors and injection list, or the
-// partials a combine stages (used before or after the tiles).
-union GatherSmem {
-    struct {
-        int anc[kTile];
-        InjList inj;
-    } t;
-    double pm[kEstN * kMarkGrid];
-    double pc[kCorrN * kGatherGrid];
+// Shared memory of k_gather: a tile's ancestors, and its injection list with the
+// first listed draw of every output.
+struct GatherSmem {
+    int anc[kTile];
+    int head[kTile];
+    InjList inj;
 };
 
 // The end of a cycle's resample on a persistent grid.  Block 0 combines
@@ -419,69 +358,25 @@ __global__ void __launch_bounds__(kThreads, 4)
              double u01_arg, const CycleArgs* ca) {
     pdl_wait();
     if (ca) gen = ca->gen;
-    __shared__ GatherSmem sm;
+    __shared__ __align__(16) GatherSmem sm;
     __shared__ int s_wmax[kThreads / 32];
     __shared__ int s_m;
     __shared__ double s_out[kEstN];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const bool resample = !cond || ctl->resample_now;
-    const bool valid = resample && ctl->w_total_fx != 0 && !ctl->w_bad;
-    if (blockIdx.x == 0) {
-        combine_staged<kEstN, kMarkGrid>(part_m, mark_grid, sm.pm, s_out);
-        double qm[4];
-        if (warp == 0) markley_mean_warp_call(&s_out[3], qm);
-        if (tid == 0) {
-            for (int q = 0; q < kEstN; ++q) ctl->est[q] = s_out[q];
-            ctl->ess = s_out[13] > 0.0 ? 1.0 / s_out[13] : 0.0;
-            ctl->est_partial = 0;
-            for (int q = 0; q < 4; ++q) ctl->qmean[q] = qm[q];
-            for (int q = 0; q < 3; ++q) ctl->cov_mean_p[q] = (float)s_out[q];
-            for (int q = 0; q < 4; ++q) ctl->cov_mean_q[q] = (float)qm[q];
-            if (resample && !valid) {
-                ctl->resample_valid = 0;
-                ctl->wmode = WMODE_UNIFORM;
-            }
-        }
-        __syncthreads();  // sm is reused by the tiles
-    }
-    if (!valid) return;
-    InjList& s_inj = sm.t.inj;
-    int* s_anc = sm.t.anc;
-    const int live = ctl->live;
-    const Offsets of = offsets(ctl, n, use_u01, u01_arg);
-    double corr[kCorrN] = {0.0, 0.0, 0.0};
-    // the tiles go to blocks 1.. (block 0 combined the sums above), or to
-    // block 0 when it is alone
+    // the tiles go to blocks 1.. (block 0 combines the sums), or to block 0 when it is
+    // alone
     const int ntiles = ceil_div(n, kTile);
     const int workers = gridDim.x > 1 ? (int)gridDim.x - 1 : 1;
     const int first = gridDim.x > 1 ? (int)blockIdx.x - 1 : 0;
-    for (int tile = first; tile >= 0 && tile < ntiles; tile += workers) {
-        const long long o0 = (long long)tile * kTile;
-        // the tile's injection draws: from its bucket, or (bucket overflow)
-        // by scanning every draw in rounds below
-        int m = 0;
-        const int cnt = k_inj > 0 ? __ldcg(&inj_cnt[tile]) : 0;
-        const bool overflow = cnt > inj_cap;
-        if (tid < kTile / 32) s_inj.hit[tid] = 0u;
-        __syncthreads();
-        if (cnt > 0 && !overflow) {
-            for (int e = tid; e < cnt; e += kThreads) {
-                const int j = __ldcg(&inj_bucket[(size_t)tile * inj_cap + e]);
-                const InjDraw d = inj_draw(of.lcg1, gen, j, n);
-                const int loc = d.idx - (int)o0;
-                s_inj.loc[e] = loc;
-                s_inj.j[e] = j;
-                s_inj.jx[e] = d.jx;
-                s_inj.jy[e] = d.jy;
-                s_inj.jz[e] = d.jz;
-                atomicOr(&s_inj.hit[loc >> 5], 1u << (loc & 31));
-            }
-            m = cnt;
+    // a tile's markers, draw count and bucket (inj_cap <= kThreads), in one round of
+    // loads; the first tile's go out together with those of the control block
+    int mk[8], cnt = 0, bj = 0;
+    auto fetch = [&](int tile) {
+        if (k_inj > 0) {
+            cnt = __ldcg(&inj_cnt[tile]);
+            if (tid < inj_cap) bj = __ldcg(&inj_bucket[(size_t)tile * inj_cap + tid]);
         }
-        // ancestors of outputs [8t, 8t + 8): running maximum of the markers
-        // (thread, then block); the markers read are reset for the next one
-        const long long i0 = o0 + 8 * tid;
-        int mk[8];
+        const long long i0 = (long long)tile * kTile + 8 * tid;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             int4 v4 = make_int4(-1, -1, -1, -1);
@@ -498,6 +393,57 @@ __global__ void __launch_bounds__(kThreads, 4)
             mk[4 * h + 2] = v4.z;
             mk[4 * h + 3] = v4.w;
         }
+    };
+    if (first >= 0 && first < ntiles) fetch(first);
+    const bool resample = !cond || ctl->resample_now;
+    const bool valid = resample && ctl->w_total_fx != 0 && !ctl->w_bad;
+    if (blockIdx.x == 0) {
+        combine_partials<kEstN, kMarkGrid, kThreads / 32>(part_m, mark_grid, s_out);
+        double qm[4];
+        if (warp == 0) markley_mean_warp_call(&s_out[3], qm);
+        if (tid == 0) {
+            for (int q = 0; q < kEstN; ++q) ctl->est[q] = s_out[q];
+            ctl->ess = s_out[13] > 0.0 ? 1.0 / s_out[13] : 0.0;
+            ctl->est_partial = 0;
+            for (int q = 0; q < 4; ++q) ctl->qmean[q] = qm[q];
+            for (int q = 0; q < 3; ++q) ctl->cov_mean_p[q] = (float)s_out[q];
+            for (int q = 0; q < 4; ++q) ctl->cov_mean_q[q] = (float)qm[q];
+            if (resample && !valid) {
+                ctl->resample_valid = 0;
+                ctl->wmode = WMODE_UNIFORM;
+            }
+        }
+    }
+    if (!valid) return;
+    InjList& s_inj = sm.inj;
+    int* s_anc = sm.anc;
+    const int live = ctl->live;
+    const uint64_t lcg1 = use_u01 ? ctl->lcg : lcg_step(ctl->lcg);
+    double corr[kCorrN] = {0.0, 0.0, 0.0};
+    for (int tile = first; tile >= 0 && tile < ntiles; tile += workers) {
+        if (tile != first) fetch(tile);
+        const long long o0 = (long long)tile * kTile;
+        // the tile's injection draws: from its bucket, or (bucket overflow)
+        // by scanning every draw in rounds below
+        const bool overflow = cnt > inj_cap;
+        const int m = overflow ? 0 : cnt;
+        if (m > 0) {
+            int4* h4 = reinterpret_cast<int4*>(sm.head);
+            h4[tid] = h4[tid + kThreads] = make_int4(-1, -1, -1, -1);
+            __syncthreads();
+            if (tid < m) {
+                const InjDraw d = inj_draw(lcg1, gen, bj, n);
+                const int loc = d.idx - (int)o0;
+                s_inj.j[tid] = bj;
+                s_inj.jx[tid] = d.jx;
+                s_inj.jy[tid] = d.jy;
+                s_inj.jz[tid] = d.jz;
+                s_inj.next[tid] = atomicExch(&sm.head[loc], tid);
+            }
+        }
+        // ancestors of outputs [8t, 8t + 8): running maximum of the markers
+        // (thread, then block); the markers read are reset for the next one
+        const long long i0 = o0 + 8 * tid;
 #pragma unroll
         for (int q = 0; q < 8; ++q)
             if (mk[q] >= 0) marker[i0 + q] = -1;
@@ -538,8 +484,13 @@ __global__ void __launch_bounds__(kThreads, 4)
             }
             // the tile's injection draws on these outputs (the bucket's, or
             // all draws in rounds on a bucket overflow)
-            if (m > 0 && ((s_inj.hit[l0 >> 5] >> (l0 & 31)) & 0xFu))
-                apply_draws(s_inj, m, l0, v[0], v[1], v[2], corr);
+            if (m > 0) {
+                const int4 hd = *reinterpret_cast<const int4*>(&sm.head[l0]);
+                if (hd.x >= 0) apply_chain(s_inj, hd.x, v[0][0], v[1][0], v[2][0], corr);
+                if (hd.y >= 0) apply_chain(s_inj, hd.y, v[0][1], v[1][1], v[2][1], corr);
+                if (hd.z >= 0) apply_chain(s_inj, hd.z, v[0][2], v[1][2], v[2][2], corr);
+                if (hd.w >= 0) apply_chain(s_inj, hd.w, v[0][3], v[1][3], v[2][3], corr);
+            }
             if (overflow) {
                 // rounds of kInjChunk draws, the round's hits on this tile
                 // compacted in draw order and applied in that order
@@ -550,7 +501,7 @@ __global__ void __launch_bounds__(kThreads, 4)
                     InjDraw d{};
                     bool hit = false;
                     if (j < k_inj) {
-                        d = inj_draw(of.lcg1, gen, j, n);
+                        d = inj_draw(lcg1, gen, j, n);
                         hit = d.idx >= o0 && d.idx < o0 + kTile;
                     }
                     const unsigned bal = __ballot_sync(~0u, hit);
@@ -596,17 +547,9 @@ __global__ void __launch_bounds__(kThreads, 4)
         if (tid == 0 && k_inj > 0) inj_cnt[tile] = 0;  // the bucket is consumed
         __syncthreads();  // s_anc and s_inj are reused by the next tile
     }
-    if (!block_partial_last<kCorrN>(corr, part_c, done)) return;
-    __threadfence();
-    combine_staged<kCorrN, kGatherGrid>(part_c, gridDim.x, sm.pc, s_out);
-    if (tid == 0) {
-        const double wd = (double)(1.0f / (float)n);
-        for (int q = 0; q < kCorrN; ++q) {
-            // block 0's sums are visible: it finished before this block
-            const double e = __ldcg(&ctl->est[q]) + wd * s_out[q];
-            ctl->est[q] = e;
-            ctl->cov_mean_p[q] = (float)e;
-        }
+    if (!block_partials_last<kCorrN, kThreads / 32>(corr, part_c, kGatherGrid, done)) return;
+    if (tid == kThreads - 1) {  // (a warp that the combine leaves idle)
+        const Offsets of = offsets(ctl, n, use_u01, u01_arg);
         ctl->lcg_next = of.lcg1;
         ctl->total_fx = of.T;
         ctl->total = of.total;
@@ -618,6 +561,14 @@ __global__ void __launch_bounds__(kThreads, 4)
         ctl->resample_valid = 1;
         ctl->wmode = WMODE_UNIFORM;
         *done = 0u;
+    }
+    combine_partials<kCorrN, kGatherGrid, kThreads / 32>(part_c, gridDim.x, s_out);
+    if (tid < kCorrN) {
+        // block 0's sums are visible: it finished before this block
+        const double wd = (double)(1.0f / (float)n);
+        const double e = __ldcg(&ctl->est[tid]) + wd * s_out[tid];
+        ctl->est[tid] = e;
+        ctl->cov_mean_p[tid] = (float)e;
     }
 }
 
