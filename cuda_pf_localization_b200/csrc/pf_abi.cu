@@ -204,8 +204,6 @@ int queue_estimate(PfHandle* h, bool sums_done = false, double skip_ratio = 0.0,
                    bool sq_from_ess = false) {
     if (!sums_done && launch_est_sums(h, sq_from_ess, skip_ratio)) return -1;
     if (launch_covs(h, false, nullptr, nullptr, false, skip_ratio)) return -1;
-    PFB_CK(cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(CycleCtl),
-                           cudaMemcpyDeviceToHost, h->stream));
     h->stats.d2h_bytes += sizeof(CycleCtl);
     PFB_CK(cudaEventRecord(h->est_ev, h->stream));
     h->est_inflight = true;
@@ -376,8 +374,8 @@ int run_cycle(PfHandle* h, const PfcOdom* odom, const CObservation* obs_dev,
     return 0;
 }
 
-// The kernels of a cycle after the predict / weighting decision, then the copy
-// of the control block.  With dargs (graph capture) the weighting pass runs
+// The kernels of a cycle after the predict / weighting decision (the last leaves the
+// control block in host memory).  With dargs (graph capture) the weighting pass runs
 // and reads its per-cycle values from dargs.
 int enqueue_cycle(PfHandle* h, const PredictArgs& pa, const CObservation* obs_dev,
                   int nobs, bool cart, const PfcCycleParams* prm, const CycleArgs* dargs) {
@@ -391,8 +389,6 @@ int enqueue_cycle(PfHandle* h, const PredictArgs& pa, const CObservation* obs_de
     if (launch_resample_est(h, prm->random_inject_ratio, true, false, 0.0, dargs))
         return -1;
     if (launch_covs(h, false, nullptr, nullptr, true)) return -1;
-    PFB_CK(cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(CycleCtl),
-                           cudaMemcpyDeviceToHost, h->stream));
     h->stats.d2h_bytes += sizeof(CycleCtl);
     // an event recorded inside a capture cannot be waited on afterwards: the
     // graph path records it after the launch
@@ -713,8 +709,6 @@ int pfc_est_sums(void* hv, double* out) {
         // covariances match the cached mean.
         if (launch_est_sums(h, true, 0.0)) return -1;
         if (launch_covs(h, false, nullptr, nullptr, false)) return -1;
-        PFB_CK(cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(CycleCtl),
-                               cudaMemcpyDeviceToHost, h->stream));
         PFB_CK(cudaStreamSynchronize(h->stream));
         h->stats.d2h_bytes += sizeof(CycleCtl);
         h->stats.host_syncs += 1;
@@ -750,8 +744,6 @@ int pfc_covs(void* hv, float mx, float my, float mz, float qw, float qx,
     if (!hit) {
         const float mp[3] = {mx, my, mz}, mq[4] = {qw, qx, qy, qz};
         if (launch_covs(h, true, mp, mq, false)) return -1;
-        PFB_CK(cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(CycleCtl),
-                               cudaMemcpyDeviceToHost, h->stream));
         PFB_CK(cudaStreamSynchronize(h->stream));
         h->stats.d2h_bytes += sizeof(CycleCtl);
         h->stats.host_syncs += 1;

@@ -127,7 +127,19 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
 }
 
-// mode: 0 plain, 1 last pass of a fused cycle (also emits the output record).
+// The control block into pinned host memory, by one block.
+__device__ __forceinline__ void control_to_host(const CycleCtl* ctl, CycleCtl* host) {
+    static_assert(sizeof(CycleCtl) % 8 == 0, "copied in words of 8 bytes");
+    __syncthreads();
+    const unsigned long long* src = reinterpret_cast<const unsigned long long*>(ctl);
+    unsigned long long* dst = reinterpret_cast<unsigned long long*>(host);
+    for (int k = threadIdx.x; k < (int)(sizeof(CycleCtl) / 8); k += kThreads) dst[k] = src[k];
+}
+
+// mode: 0 plain, 1 last pass of a fused cycle (also emits the output record).  The
+// last block (or, skipping, the first) leaves the control block in host memory for
+// the caller, which waits for the kernel: a cycle of 4096 particles takes 49 us so,
+// 56 with a copy queued behind it.
 // skip_ratio > 0: the caller resamples whenever the ESS of the estimate just
 // computed is below skip_ratio * n (ParticleFilter::update's rule), and then
 // discards this estimate's covariances; the pass is skipped in that case and
@@ -136,10 +148,13 @@ __global__ void __launch_bounds__(kThreads, 2)
     k_covs(PlaneSet ps, int n, const float* __restrict__ ll,
            const float* __restrict__ w, double* part, unsigned* done,
            CycleCtl* ctl, int use_args, float3 mp_arg, float4 mq_arg,
-           int mode, double skip_ratio) {
+           int mode, double skip_ratio, CycleCtl* host) {
     pdl_wait();
     if (skip_ratio > 0.0 && ctl->ess < skip_ratio * (double)n) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->cov_mean_p[0] = __int_as_float(0x7fc00000);
+        if (blockIdx.x == 0) {
+            if (threadIdx.x == 0) ctl->cov_mean_p[0] = __int_as_float(0x7fc00000);
+            control_to_host(ctl, host);
+        }
         return;
     }
     const Planes s = pick_planes(ps, ctl->live);
@@ -216,6 +231,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             o[PFC_EST_RESAMPLED] = ctl->resampled ? 1.0 : 0.0;
         }
     }
+    control_to_host(ctl, host);
 }
 
 // Weight pass before a resample: weights materialised from the
@@ -427,7 +443,7 @@ int launch_covs(PfHandle* h, bool use_args, const float mp[3],
     KernelScope ks(h, KK_COVS);
     PFB_CK(launch_pdl(k_covs, est_grid(h->n), kThreads, 0, h->stream, plane_set(h), h->n,
                       h->d_ll, h->d_w, h->d_part, h->d_done + 2, h->d_ctl,
-                      use_args ? 1 : 0, a, b, cycle_output ? 1 : 0, skip_ratio));
+                      use_args ? 1 : 0, a, b, cycle_output ? 1 : 0, skip_ratio, h->h_ctl));
     PFB_KL();
     return 0;
 }
