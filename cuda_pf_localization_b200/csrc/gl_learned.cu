@@ -79,12 +79,14 @@ enum Epi : int {
     EPI_F32 = 3,         // f32 acc * scale, row-major
 };
 
+struct Mat;
 struct EpiArgs {
-    void* out;
-    void* outT;         // transposed copy (bf16 epilogues; may be null)
-    const float* bias;  // [N]
-    const bf16* mask;   // [M][ldm] activations whose sign gates the gradient
-    int ldo, ldt, ldm;
+    float* out;            // f32 epilogues: row-major output, ldo columns
+    const Mat *mo, *mt;    // bf16 epilogues: the output and its transpose (host only)
+    const float* bias;     // [N]
+    uint32_t* bits;        // relu' of the activations: word [N / 32][ldb rows], see below
+    int transpose;         // whether the transposed output is written
+    int ldo, ldb;
     float scale;
     long long split_stride;  // f32 elements between split-K partial outputs
 };
@@ -95,22 +97,41 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
 }
 
 // Epilogue of one warp's 32 rows x 32 columns at (row0, col0): lane l arrives with
-// row row0 + l.  The chunk passes through 4 KiB of shared memory and leaves in
-// 16-byte pieces, of which four lanes (bf16) or eight (f32) fill a 64- or 128-byte
-// line segment of the output, and of the transposed one.  Stored from the registers
-// as they are, each lane writes 16 bytes of its own row at a time, half a sector,
-// and two bytes a column of the transpose: the epilogue, not the MMAs, then bounds a
-// tile (26 of a launch's 38 thousand cycles).  Training step, so stored and as here:
-// 389 and 355 us at a batch of 8192, 210 and 200 at 2048, 181 and 172 at 512 (CTA
-// pairs with 256 x 256 tiles were slower than this, 364 at 8192).
-// m: the chunk's mask words (relu' gating).
+// row row0 + l.  The chunk passes through the warp's 4 KiB of shared memory: f32
+// outputs leave in 16-byte pieces of which eight lanes fill a 128-byte line, bf16
+// ones, row-major and transposed, by a TMA store each (the 64-byte swizzle of its map
+// keeps the lanes' pieces on different banks).
+//
+// What bounds a tile is the load/store unit: stored from the registers as they are, a
+// lane writes 16 bytes of its own row at a time and two bytes a column of the
+// transpose, 26 thousand cycles a launch of 256 tiles; through shared memory in
+// 16-byte pieces, with the activations read for the backward gate, about 280 cycles
+// a chunk, 9 thousand a tile where the MMAs take 8; like this about 60.  The gate
+// of the backward pass, relu'(z) = 1 exactly when the stored activation is > 0, is a
+// word of bits per row and chunk that the forward pass leaves: bit 15 - k for
+// column 2k, 31 - k for column 2k + 1.  Training step, registers, pieces and this:
+// 389, 355 and 331 us at a batch of 8192, 210, 200 and 194 at 2048, 181, 172 and 165
+// at 512.
 constexpr int kStagedBytes = 4096;  // of an epilogue warp
 template <int EPI>
-__device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[32], const uint4 (&m)[4],
-                                               int row0, int col0, const float* bias,
-                                               const EpiArgs& ep, unsigned char* stage) {
+__device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[32], uint32_t gate,
+                                               const CUtensorMap* tmO, const CUtensorMap* tmT,
+                                               int row0, int col0, const EpiArgs& ep,
+                                               unsigned char* stage) {
     const int lane = threadIdx.x & 31;
     uint4* rows = reinterpret_cast<uint4*>(stage);  // [row][pieces], swizzled
+    float bias[32];
+    if constexpr (EPI == EPI_BIAS_F32 || EPI == EPI_RELU_BF16) {
+        const float4* b4 = reinterpret_cast<const float4*>(ep.bias + col0);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const float4 b = __ldg(&b4[q]);
+            bias[4 * q] = b.x;
+            bias[4 * q + 1] = b.y;
+            bias[4 * q + 2] = b.z;
+            bias[4 * q + 3] = b.w;
+        }
+    }
     if constexpr (EPI == EPI_F32 || EPI == EPI_BIAS_F32) {
         const float s = EPI == EPI_F32 ? ep.scale : 1.0f;
         auto value = [&](int j) {
@@ -124,14 +145,15 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[32], const ui
                                                            value(4 * q + 2), value(4 * q + 3));
         __syncwarp();
         const int line = lane >> 3, piece = lane & 7;
-        float* out = reinterpret_cast<float*>(ep.out) + (size_t)row0 * ep.ldo + col0 + 4 * piece;
+        float* out = ep.out + (size_t)row0 * ep.ldo + col0 + 4 * piece;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int x = 4 * i + line;
             *reinterpret_cast<uint4*>(out + (size_t)x * ep.ldo) = rows[8 * x + (piece ^ (x & 7))];
         }
+        __syncwarp();  // the stage is reused
     } else {
-        uint32_t w[16];  // columns (2k, 2k + 1) of row `lane`
+        uint32_t w[16], bits = 0;  // columns (2k, 2k + 1) of row `lane`
 #pragma unroll
         for (int k = 0; k < 16; ++k) {
             float a = __uint_as_float(r[2 * k]), b = __uint_as_float(r[2 * k + 1]);
@@ -139,86 +161,84 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[32], const ui
                 a = fmaxf(a + bias[2 * k], 0.0f);
                 b = fmaxf(b + bias[2 * k + 1], 0.0f);
             } else {
-                const uint4 u = m[k / 4];
-                const uint32_t x = k % 4 == 0 ? u.x : k % 4 == 1 ? u.y : k % 4 == 2 ? u.z : u.w;
-                // relu'(z) = 1 exactly when the stored activation is > 0
-                if ((int)(short)(x & 0xFFFFu) <= 0) a = 0.0f;
-                if ((int)(short)(x >> 16) <= 0) b = 0.0f;
+                if (!(gate & (0x8000u >> k))) a = 0.0f;
+                if (!(gate & (0x80000000u >> k))) b = 0.0f;
             }
             w[k] = pack_bf16x2(a, b);
+            // the halves are >= 0 (or -0): adding 0x7FFF carries into the sign of the
+            // ones that are not 0
+            if (EPI == EPI_RELU_BF16)
+                bits |= ((w[k] + 0x7FFF7FFFu) & ~w[k] & 0x80008000u) >> k;
         }
-        uint32_t* cols = reinterpret_cast<uint32_t*>(stage + 2048);  // [column][16 row pairs]
+        if (EPI == EPI_RELU_BF16 && ep.bits)
+            ep.bits[(size_t)(col0 >> 5) * ep.ldb + row0 + lane] = bits;
+        if (lane == 0) bulk_wait_read();  // the chunk before has left the stage
+        __syncwarp();
+        uint32_t* cols = reinterpret_cast<uint32_t*>(stage + 2048);  // [column][row pairs]
         const int sw = (lane >> 1) & 3;
 #pragma unroll
         for (int q = 0; q < 4; ++q)
             rows[4 * lane + (q ^ sw)] =
                 make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-        if (ep.outT) {
+        if (ep.transpose) {
             // even lanes take the even columns of their row and the next, odd lanes
             // the odd ones
             const bool odd = lane & 1;
+            const int at = (lane & 1) * 16 + sw;
 #pragma unroll
             for (int k = 0; k < 16; ++k) {
                 const uint32_t o = __shfl_xor_sync(~0u, w[k], 1);
-                cols[(2 * k + (lane & 1)) * 16 + (lane >> 1)] =
+                cols[32 * k + at + 4 * ((lane >> 3) ^ (k & 3))] =
                     odd ? __byte_perm(o, w[k], 0x7632) : __byte_perm(w[k], o, 0x5410);
             }
         }
+        fence_async_shared();
         __syncwarp();
-        const int line = lane >> 2, piece = lane & 3;
-        bf16* out = reinterpret_cast<bf16*>(ep.out) + (size_t)row0 * ep.ldo + col0 + 8 * piece;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int x = 8 * i + line;
-            *reinterpret_cast<uint4*>(out + (size_t)x * ep.ldo) =
-                rows[4 * x + (piece ^ ((x >> 1) & 3))];
-        }
-        if (ep.outT) {
-            bf16* outT = reinterpret_cast<bf16*>(ep.outT) + (size_t)col0 * ep.ldt + row0 + 8 * piece;
-            const uint4* c4 = reinterpret_cast<const uint4*>(cols);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int x = 8 * i + line;
-                *reinterpret_cast<uint4*>(outT + (size_t)x * ep.ldt) = c4[4 * x + piece];
-            }
+        if (lane == 0) {
+            tma_store_2d(tmO, rows, col0, row0);
+            if (ep.transpose) tma_store_2d(tmT, cols, row0, col0);
+            bulk_commit();
         }
     }
-    __syncwarp();  // the stage is reused
 }
 
-// One epilogue warp's chunks part, part + kPerQ, ... of its 32 rows of a tile, with
-// the mask of each loaded while the one before is stored.  last(): called once the
-// accumulator has been read.
-template <int EPI, int kChunks, int kPerQ, class Last>
-__device__ __forceinline__ void epilogue_tile(uint32_t trow, int row0, int n0, int part,
-                                              const EpiArgs& ep, unsigned char* stage,
-                                              Last last) {
-    const int lane = threadIdx.x & 31;
-    uint4 mask[4] = {}, next[4] = {};
-    auto load_mask = [&](int c) {
-        if constexpr (EPI == EPI_DRELU_BF16) {
-            const uint4* mp = reinterpret_cast<const uint4*>(
-                ep.mask + (size_t)(row0 + lane) * ep.ldm + n0 + c * 32);
+// The words of one epilogue warp's chunks (gates of the backward pass).
+template <int EPI, int kMine, int kPerQ>
+__device__ __forceinline__ void load_gates(uint32_t (&g)[kMine], int row0, int n0, int part,
+                                           const EpiArgs& ep) {
+    if constexpr (EPI == EPI_DRELU_BF16) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) next[k] = mp[k];
-        }
-    };
-    load_mask(part);
+        for (int i = 0; i < kMine; ++i)
+            g[i] = __ldg(&ep.bits[(size_t)((n0 >> 5) + part + i * kPerQ) * ep.ldb + row0 +
+                                  (threadIdx.x & 31)]);
+    }
+}
+
+// One epilogue warp's chunks part, part + kPerQ, ... of its 32 rows of a tile.
+// last(): called once the accumulator has been read.
+template <int EPI, int kMine, int kPerQ, class Last>
+__device__ __forceinline__ void epilogue_tile(uint32_t trow, const uint32_t (&gates)[kMine],
+                                              const CUtensorMap* tmO, const CUtensorMap* tmT,
+                                              int row0, int n0, int part, const EpiArgs& ep,
+                                              unsigned char* stage, Last last) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll 1
-    for (int c = part; c < kChunks; c += kPerQ) {
+    for (int i = 0; i < kMine; ++i) {
+        const int c = part + i * kPerQ;
         uint32_t v[32];
         tmem_ld32(trow + (uint32_t)(c * 32), v);
+        uint32_t gate = 0;
+        if (EPI == EPI_DRELU_BF16) {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) mask[k] = next[k];
-        if (c + kPerQ < kChunks) load_mask(c + kPerQ);
+            for (int k = 0; k < kMine; ++k) gate = i == k ? gates[k] : gate;
+        }
         tmem_wait_ld();
-        if (c + kPerQ >= kChunks) {  // this warp's last chunk: hand it back
+        if (i == kMine - 1) {  // this warp's last chunk: hand it back
             tc_fence_before();
             __syncwarp();
             if (lane == 0) last();
         }
-        epilogue_chunk<EPI>(v, mask, row0, n0 + c * 32,
-                            ep.bias ? ep.bias + n0 + c * 32 : nullptr, ep, stage);
+        epilogue_chunk<EPI>(v, gate, tmO, tmT, row0, n0 + c * 32, ep, stage);
     }
 }
 
@@ -263,7 +283,9 @@ struct TileGrid {
 template <int EPI, int BN>
 __global__ void __launch_bounds__(kPThreads, 1)
     k_gemm_bf16_ws(const __grid_constant__ CUtensorMap tmA,
-                   const __grid_constant__ CUtensorMap tmB, int K, int a_row0,
+                   const __grid_constant__ CUtensorMap tmB,
+                   const __grid_constant__ CUtensorMap tmO,
+                   const __grid_constant__ CUtensorMap tmT, int K, int a_row0,
                    int a_k0, int b_row0, int b_k0, TileGrid tg, EpiArgs ep,
                    unsigned* __restrict__ err) {
     constexpr int S = PTile<BN>::kStages;
@@ -395,12 +417,14 @@ __global__ void __launch_bounds__(kPThreads, 1)
         const int q = warp & 3;
         constexpr int kPerQ = kEpiWarps / 4;  // warps sharing a lane quarter
         const int part = (warp - 2) / 4;      // which of them: chunks part, part + kPerQ, ...
-        constexpr int kChunks = BN / 32;
+        constexpr int kMine = BN / 32 / kPerQ;
         int i = 0;
         for (int t = blockIdx.x; t < tg.tiles; t += gridDim.x, ++i) {
             const int z = t / tg.tmn, r = t - z * tg.tmn;
             const int m0 = (r / tg.tn) * BM, n0 = (r % tg.tn) * BN;
             const int b = i & 1, use = i >> 1;
+            uint32_t gates[kMine];
+            load_gates<EPI, kMine, kPerQ>(gates, m0 + q * 32, n0, part, ep);
             const bool got = __all_sync(
                 ~0u, mbar_wait_abort(&acc_full[b], use & 1, kWaitLimit, abort));
             if (!got) {
@@ -413,12 +437,13 @@ __global__ void __launch_bounds__(kPThreads, 1)
             tc_fence_after();
             EpiArgs et = ep;
             if (EPI == EPI_F32)
-                et.out = reinterpret_cast<float*>(ep.out) + (size_t)z * ep.split_stride;
+                et.out = ep.out + (size_t)z * ep.split_stride;
             const uint32_t trow = tmem + (uint32_t)(b * BN) + ((uint32_t)(q * 32) << 16);
-            epilogue_tile<EPI, kChunks, kPerQ>(trow, m0 + q * 32, n0, part, et,
-                                               staged + (warp - 2) * kStagedBytes,
-                                               [&] { mbar_arrive(&acc_empty[b]); });
+            epilogue_tile<EPI, kMine, kPerQ>(trow, gates, &tmO, &tmT, m0 + q * 32, n0, part, et,
+                                             staged + (warp - 2) * kStagedBytes,
+                                             [&] { mbar_arrive(&acc_empty[b]); });
         }
+        if (lane == 0) bulk_wait();  // the stores are complete before the CTA ends
     }
     tc_fence_before();
     __syncthreads();
@@ -450,10 +475,10 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// Tensor map of a row-major rows x cols bf16 matrix with box_rows x 64 boxes
-// and the 128-byte swizzle.
+// Tensor map of a row-major rows x cols bf16 matrix with box_rows x box_cols boxes
+// and the swizzle of a box row's length.
 int make_map(CUtensorMap* m, const void* ptr, long long rows, long long cols,
-             int box_rows) {
+             int box_rows, int box_cols = BK) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) {
         set_error("pf_b200: cuTensorMapEncodeTiled is unavailable");
@@ -465,12 +490,13 @@ int make_map(CUtensorMap* m, const void* ptr, long long rows, long long cols,
     }
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
     const cuuint32_t es[2] = {1, 1};
     const CUresult r =
         fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims,
            strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+           box_cols == BK ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+           CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         set_error("pf_b200: cuTensorMapEncodeTiled failed (%d)", (int)r);
@@ -479,15 +505,16 @@ int make_map(CUtensorMap* m, const void* ptr, long long rows, long long cols,
     return 0;
 }
 
-// A bf16 matrix as a GEMM operand: tensor maps with 128-row and (when the
-// matrix has at least 256 rows) 256-row boxes.
+// A bf16 matrix as a GEMM operand or output: tensor maps with 128-row and (when the
+// matrix has at least 256 rows) 256-row boxes to load, and 32 x 32 ones to store.
 struct Mat {
-    CUtensorMap m128, m256;
+    CUtensorMap m128, m256, store;
     bool has256 = false;
 };
 
 int make_mat(Mat* m, const void* ptr, long long rows, long long cols) {
     if (make_map(&m->m128, ptr, rows, cols, 128)) return -1;
+    if (make_map(&m->store, ptr, rows, cols, 32, 32)) return -1;
     m->has256 = rows >= 256;
     if (m->has256 && make_map(&m->m256, ptr, rows, cols, 256)) return -1;
     return 0;
@@ -526,18 +553,21 @@ int gemm_bn(cudaStream_t s, MapRef a, MapRef b, int M, int N, int K,
     tg.splits = splits;
     const int grid = std::min(tg.tiles, sm_count());
     const CUtensorMap& tb = BN == 256 ? b.map->m256 : b.map->m128;
-    PFB_CK(launch_pdl(k_gemm_bf16_ws<EPI, BN>, grid, kPThreads, smem, s, a.map->m128, tb, K,
-                      a.row0, a.k0, b.row0, b.k0, tg, ep, err));
+    const Mat* mo = ep.mo ? ep.mo : a.map;  // (f32 outputs use neither store map)
+    const Mat* mt = ep.mt ? ep.mt : a.map;
+    PFB_CK(launch_pdl(k_gemm_bf16_ws<EPI, BN>, grid, kPThreads, smem, s, a.map->m128, tb,
+                      mo->store, mt->store, K, a.row0, a.k0, b.row0, b.k0, tg, ep, err));
     PFB_KL();
     return 0;
 }
 
 // D = A B^T.  The 128 x 256 tile is used when N allows it and there are more 128 x
 // 128 tiles than SMs: a round of wide tiles takes about one and a half of narrow
-// ones.  Training step with wide and with narrow tiles in the layers this decides:
-// 244 and 256 us at a batch of 4096 (128 or 256 tiles), 308 and 307 at 4864 (152 or
-// 304), 355 and 393 at 8192, 584 and 621 at 16384; 226 and 200 at 2048 (64 or 128,
-// narrow).  Both sum k in the same order: the results are the same bits.
+// ones.  Training step with wide and with narrow tiles in the layers this decides
+// (before the epilogues stored by TMA): 244 and 256 us at a batch of 4096 (128 or 256
+// tiles), 308 and 307 at 4864 (152 or 304), 355 and 393 at 8192, 584 and 621 at 16384;
+// 226 and 200 at 2048 (64 or 128, narrow).  Both sum k in the same order: the results
+// are the same bits.
 template <int EPI>
 int gemm(cudaStream_t s, MapRef a, MapRef b, int M, int N, int K,
          const EpiArgs& ep, unsigned* err, int splits = 1) {
@@ -1156,6 +1186,7 @@ struct LpHandle {
     Layer L[kLayers];
     bf16* H[kLayers - 1] = {};
     bf16* HT[kLayers - 1] = {};
+    uint32_t* gate[kLayers - 1] = {};  // relu' bits of H
     bf16* dZ[kLayers] = {};
     bf16* dZT[kLayers] = {};
     float* Z4 = nullptr;
@@ -1261,11 +1292,14 @@ int forward(LpHandle* h, MapRef x, int rows, bool write_t) {
     cudaStream_t s = h->stream;
     for (int l = 0; l < kLayers - 1; ++l) {
         EpiArgs ep{};
-        ep.out = h->H[l];
-        ep.outT = write_t ? h->HT[l] : nullptr;
+        ep.mo = &h->tm_H[l];
         ep.bias = h->L[l].b;
-        ep.ldo = h->L[l].out;
-        ep.ldt = h->batch;
+        if (write_t) {
+            ep.mt = &h->tm_HT[l];
+            ep.transpose = 1;
+            ep.bits = h->gate[l];
+            ep.ldb = h->batch;
+        }
         const MapRef a = l == 0 ? x : MapRef{&h->tm_H[l - 1], 0, 0};
         if (gemm<EPI_RELU_BF16>(s, a, MapRef{&h->L[l].tm_w, 0, 0}, rows,
                                 h->L[l].out, h->L[l].in, ep, h->d_err))
@@ -1323,12 +1357,11 @@ int backward(LpHandle* h, MapRef xt, const float* Y, float* d_loss_slot) {
             return -1;
         if (l > 0) {
             EpiArgs ed{};
-            ed.out = h->dZ[l - 1];
-            ed.outT = h->dZT[l - 1];
-            ed.mask = h->H[l - 1];
-            ed.ldo = L.in;
-            ed.ldt = B;
-            ed.ldm = L.in;
+            ed.mo = &h->tm_dZ[l - 1];
+            ed.mt = &h->tm_dZT[l - 1];
+            ed.transpose = 1;
+            ed.bits = h->gate[l - 1];
+            ed.ldb = B;
             if (gemm<EPI_DRELU_BF16>(s, MapRef{&h->tm_dZ[l], 0, 0},
                                      MapRef{&L.tm_wt, 0, 0}, B, L.in, L.out, ed,
                                      h->d_err))
@@ -1393,6 +1426,7 @@ void free_lp(LpHandle* h) {
     for (int l = 0; l < kLayers - 1; ++l) {
         cudaFree(h->H[l]);
         cudaFree(h->HT[l]);
+        cudaFree(h->gate[l]);
     }
     cudaFree(h->Z4);
     cudaFree(h->X);
@@ -1701,6 +1735,7 @@ void* pfgl_learned_create(void* glv, int batch, unsigned long long seed) {
         for (int l = 0; l < kLayers - 1 && !bad; ++l) {
             bad = dalloc(&h->H[l], (size_t)batch * kHid) ||
                   dalloc(&h->HT[l], (size_t)batch * kHid) ||
+                  dalloc(&h->gate[l], (size_t)batch * kHid / 32) ||
                   make_mat(&h->tm_H[l], h->H[l], batch, kHid) ||
                   make_mat(&h->tm_HT[l], h->HT[l], kHid, batch);
         }
