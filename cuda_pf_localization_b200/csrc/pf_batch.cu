@@ -93,7 +93,6 @@ struct BGlobal {
     unsigned scan_epoch;
     unsigned inj_epoch;
     unsigned tile_counter;
-    unsigned err;
     // look-back polls before a wait gives up (kSpinLimit unless the host
     // lowers it), and the filter whose first resampling tile publishes its
     // prefix under a stale epoch (-1: none), so that the waits of its later
@@ -132,7 +131,6 @@ __global__ void k_b_init(BCtl* C, BGlobal* G, int nf) {
         G->scan_epoch = 1u;
         G->inj_epoch = 1u;
         G->tile_counter = 0u;
-        G->err = 0u;
         G->spin_limit = kSpinLimit;
         G->stall_f = -1;
     }
@@ -358,7 +356,7 @@ __device__ __forceinline__ void ess_span(const float* __restrict__ ll, float* __
 __global__ void __launch_bounds__(kThreads)
     k_b_ess(Arena A, const BFilter* __restrict__ F, const BTile* __restrict__ T,
             BCtl* C, double* __restrict__ epart,
-            unsigned long long* __restrict__ eupart, double* __restrict__ out) {
+            unsigned long long* __restrict__ eupart) {
     const BTile t = T[blockIdx.x];
     const BFilter& fl = F[t.f];
     BCtl* c = C + t.f;
@@ -411,11 +409,8 @@ __global__ void __launch_bounds__(kThreads)
         const double ess = sq > 0.0 ? 1.0 / sq : 0.0;
         c->ess = ess;
         c->ess_pre = ess;
-        double* o = out + (size_t)t.f * PFC_EST_LEN;
-        o[PFC_EST_ESS_PRE] = ess;
         c->resample_now = (fl.ess_ratio > 0.0 && ess < fl.ess_ratio * (double)fl.n) ? 1 : 0;
         c->resampled = 0;
-        o[PFC_EST_RESAMPLED] = 0.0;
         c->w_total_fx = tot;
         c->w_bad = any_fb ? 1 : 0;
         if (wmode == WMODE_LL) c->wmode = WMODE_STORED;
@@ -496,11 +491,13 @@ __global__ void __launch_bounds__(kThreads, 3)
     }
 }
 
-// Covariance pass and the filter's output record.  Three blocks per SM, as
-// the estimate pass (1.788 against 1.799 ms per 512-filter cycle at two).
+// Covariance pass and the filter's output record, which goes straight to pinned host
+// memory with the filter's error bits, as no copy has to follow the kernel then.
+// Three blocks per SM, as the estimate pass (1.788 against 1.799 ms per 512-filter
+// cycle at two).
 __global__ void __launch_bounds__(kThreads, 3)
     k_b_covs(Arena A, const BFilter* __restrict__ F, const BTile* __restrict__ T,
-             BCtl* C, double* __restrict__ cpart, double* __restrict__ out) {
+             BCtl* C, double* __restrict__ cpart, double* out, unsigned* host_err) {
     const BTile t = T[blockIdx.x];
     const BFilter& fl = F[t.f];
     BCtl* c = C + t.f;
@@ -551,9 +548,10 @@ __global__ void __launch_bounds__(kThreads, 3)
         return;
     __shared__ double s_out[kCovN];
     tiles_combine<kCovN>(cpart + (size_t)fl.etile0 * kCovN, fl.netiles, s_out);
+    __shared__ double s_rec[PFC_EST_LEN];
     if (threadIdx.x == 0) {
         for (int k = 0; k < kCovN; ++k) c->covs[k] = s_out[k];
-        double* o = out + (size_t)t.f * PFC_EST_LEN;
+        double* o = s_rec;
         for (int k = 0; k < 3; ++k) o[PFC_EST_POS + k] = c->est[k];
         for (int k = 0; k < 4; ++k) o[PFC_EST_QUAT + k] = c->qmean[k];
         for (int k = 0; k < 6; ++k) o[PFC_EST_POSCOV + k] = s_out[k];
@@ -561,9 +559,14 @@ __global__ void __launch_bounds__(kThreads, 3)
         // without a resample the record carries the ESS the decision used,
         // as ParticleFilter::update returns its first estimate
         o[PFC_EST_ESS] = c->resampled ? c->ess : c->ess_pre;
+        o[PFC_EST_ESS_PRE] = c->ess_pre;
         o[PFC_EST_RESAMPLED] = c->resampled ? 1.0 : 0.0;
+        if (c->err) atomicOr_system(host_err, c->err);
         c->done_c = 0u;
     }
+    __syncthreads();
+    if (threadIdx.x <= PFC_EST_ESS_PRE)
+        out[(size_t)t.f * PFC_EST_LEN + threadIdx.x] = s_rec[threadIdx.x];
 }
 
 // Resampling of one 4096-particle tile of a filter that resamples: the
@@ -903,7 +906,6 @@ __global__ void __launch_bounds__(kThreads)
             }
             c->wmode = WMODE_UNIFORM;
         }
-        if (c->err) atomicOr(&G->err, c->err);
         if (blockIdx.x == 0) {
             G->tile_counter = 0u;
             unsigned e = (G->scan_epoch + 1u) & 0x3FFFFFFFu;
@@ -987,7 +989,7 @@ struct BatchHandle {
     int n_rt = 0;
     BCtl* d_C = nullptr;
     BGlobal* d_G = nullptr;
-    BGlobal* h_G = nullptr;
+    unsigned* h_err = nullptr;       // pinned; error bits of every filter so far
     float2* d_wpart = nullptr;
     double* d_epart = nullptr;
     unsigned long long* d_eupart = nullptr;
@@ -1010,8 +1012,7 @@ struct BatchHandle {
     CObservation* d_obs = nullptr;
     CObservation* h_obs = nullptr;   // pinned
     int obs_cap = 0;
-    double* d_out = nullptr;
-    double* h_out = nullptr;         // pinned
+    double* h_out = nullptr;         // pinned, written by k_b_covs
     float* d_prior = nullptr;
     float* d_tmp = nullptr;
     long long tmp_cap = 0;
@@ -1091,7 +1092,7 @@ int launch_est_covs(BatchHandle* h) {
     PFB_CK(launch_pdl(k_b_est, h->n_et, kThreads, 0, h->stream, h->A, h->d_F, h->d_et, h->d_C,
                       h->d_epart));
     PFB_CK(launch_pdl(k_b_covs, h->n_et, kThreads, 0, h->stream, h->A, h->d_F, h->d_et, h->d_C,
-                      h->d_cpart, h->d_out));
+                      h->d_cpart, h->h_out, h->h_err));
     h->launches += 2;
     PFB_KL();
     return 0;
@@ -1104,7 +1105,7 @@ int enqueue_cycle(BatchHandle* h) {
     PFB_CK(launch_pdl(k_b_weight, h->n_wt, kWThreads, 0, s, h->A, h->d_F, h->d_wt, h->d_C,
                       h->d_cyc, h->d_obs, h->d_lm, h->d_wpart, h->use_packed));
     PFB_CK(launch_pdl(k_b_ess, h->n_et, kThreads, 0, s, h->A, h->d_F, h->d_et, h->d_C,
-                      h->d_epart, h->d_eupart, h->d_out));
+                      h->d_epart, h->d_eupart));
     PFB_CK(launch_pdl(k_b_resample, h->n_rt, kThreads, 0, s, h->A, h->d_F, h->d_rt, h->d_C,
                       h->d_G, h->d_flags, h->d_vals));
     PFB_CK(launch_pdl(k_b_gather, h->n_gt, kThreads, 0, s, h->A, h->d_F, h->d_gt, h->d_C,
@@ -1124,7 +1125,6 @@ int enqueue_cycle(BatchHandle* h) {
     h->launches += 1;
     PFB_KL();
     if (launch_est_covs(h)) return -1;
-    PFB_CK(cudaMemcpyAsync(h->h_G, h->d_G, sizeof(BGlobal), cudaMemcpyDeviceToHost, s));
     return 0;
 }
 
@@ -1152,12 +1152,8 @@ int run_cycle(BatchHandle* h) {
 }
 
 int finish(BatchHandle* h, double* est_out) {
-    if (est_out)
-        PFB_CK(cudaMemcpyAsync(h->h_out, h->d_out,
-                               sizeof(double) * PFC_EST_LEN * (size_t)h->nf,
-                               cudaMemcpyDeviceToHost, h->stream));
     PFB_CK(cudaStreamSynchronize(h->stream));
-    if (h->h_G->err & ERR_SPIN_TIMEOUT) {
+    if (*h->h_err & ERR_SPIN_TIMEOUT) {
         set_error("pf_b200: batch look-back wait timed out");
         return -1;
     }
@@ -1177,7 +1173,7 @@ void free_batch(BatchHandle* h) {
     cudaFree(h->d_rt);
     cudaFree(h->d_C);
     cudaFree(h->d_G);
-    cudaFreeHost(h->h_G);
+    cudaFreeHost(h->h_err);
     cudaFree(h->d_wpart);
     cudaFree(h->d_epart);
     cudaFree(h->d_eupart);
@@ -1196,7 +1192,6 @@ void free_batch(BatchHandle* h) {
     cudaFreeHost(h->h_cyc);
     cudaFree(h->d_obs);
     cudaFreeHost(h->h_obs);
-    cudaFree(h->d_out);
     cudaFreeHost(h->h_out);
     cudaFree(h->d_prior);
     cudaFree(h->d_tmp);
@@ -1286,7 +1281,7 @@ void* pfc_batch_create(int n_filters, const int* n, const unsigned* seeds,
             cudaMalloc((void**)&h->d_rt, sizeof(BTile) * rt.size()) != cudaSuccess ||
             cudaMalloc((void**)&h->d_C, sizeof(BCtl) * n_filters) != cudaSuccess ||
             cudaMalloc((void**)&h->d_G, sizeof(BGlobal)) != cudaSuccess ||
-            cudaMallocHost((void**)&h->h_G, sizeof(BGlobal)) != cudaSuccess ||
+            cudaMallocHost((void**)&h->h_err, sizeof(unsigned)) != cudaSuccess ||
             cudaMalloc((void**)&h->d_wpart, sizeof(float2) * wt.size()) != cudaSuccess ||
             cudaMalloc((void**)&h->d_flags, sizeof(unsigned) * rt.size()) != cudaSuccess ||
             cudaMalloc((void**)&h->d_vals, sizeof(uint64_t) * 2 * rt.size()) != cudaSuccess)
@@ -1311,13 +1306,12 @@ void* pfc_batch_create(int n_filters, const int* n, const unsigned* seeds,
             cudaMallocHost((void**)&h->h_cyc, sizeof(PfcBatchCycle) * n_filters) != cudaSuccess ||
             cudaMalloc((void**)&h->d_obs, sizeof(CObservation) * h->obs_cap) != cudaSuccess ||
             cudaMallocHost((void**)&h->h_obs, sizeof(CObservation) * h->obs_cap) != cudaSuccess ||
-            cudaMalloc((void**)&h->d_out, sizeof(double) * PFC_EST_LEN * n_filters) != cudaSuccess ||
             cudaMallocHost((void**)&h->h_out, sizeof(double) * PFC_EST_LEN * n_filters) != cudaSuccess ||
             cudaMalloc((void**)&h->d_prior, sizeof(float) * 13 * n_filters) != cudaSuccess)
             break;
-        if (cudaMemset(h->d_cyc, 0, sizeof(PfcBatchCycle) * n_filters) != cudaSuccess ||
-            cudaMemset(h->d_out, 0, sizeof(double) * PFC_EST_LEN * n_filters) != cudaSuccess)
-            break;
+        if (cudaMemset(h->d_cyc, 0, sizeof(PfcBatchCycle) * n_filters) != cudaSuccess) break;
+        memset(h->h_out, 0, sizeof(double) * PFC_EST_LEN * n_filters);
+        *h->h_err = 0u;
         // an empty landmark table until landmarks are uploaded
         if (cudaMalloc((void**)&h->d_lm, sizeof(float) * 3) != cudaSuccess) break;
         if (cudaMemcpy(h->d_wt, wt.data(), sizeof(BTile) * wt.size(),
