@@ -813,10 +813,12 @@ const uint64_t* small_select(GlHandle* h, const float* caer, const uint64_t* key
     return out;
 }
 
+// With host set the entries also go to pinned host memory: a call that waits for the
+// kernel then needs no copies behind it (three to pageable memory cost 30 us).
 __global__ void k_gather_topk(const uint64_t* __restrict__ keys, int k,
                               const float* __restrict__ hyp,
                               const float* __restrict__ caer, float* out3,
-                              float* outc, int* outi) {
+                              float* outc, int* outi, TopHost* host) {
     const int j = blockIdx.x * kThreads + threadIdx.x;
     if (j >= k) return;
     const int src = (int)(uint32_t)keys[j];
@@ -825,6 +827,11 @@ __global__ void k_gather_topk(const uint64_t* __restrict__ keys, int k,
     out3[3 * j + 2] = hyp[3 * src + 2];
     outc[j] = caer[src];
     outi[j] = src;
+    if (host) {
+        for (int q = 0; q < 3; ++q) host->pose[3 * j + q] = hyp[3 * src + q];
+        host->caer[j] = caer[src];
+        host->idx[j] = src;
+    }
 }
 
 // Bottom-k of many queries: out[q * k + j] from key q * k + j, whose index
@@ -1004,20 +1011,28 @@ const uint64_t* smallest_current(GlHandle* h, int k) {
 
 int copy_topk(GlHandle* h, const uint64_t* sorted, int k, float* out3k,
               float* caer_k, int* idx_k) {
+    TopHost* host = k <= TopHost::kTop ? h->h_top : nullptr;
     k_gather_topk<<<ceil_div(k, kThreads), kThreads, 0, h->stream>>>(
-        sorted, k, h->d_hyp, h->d_caer, h->d_out, h->d_outc, h->d_outi);
+        sorted, k, h->d_hyp, h->d_caer, h->d_out, h->d_outc, h->d_outi, host);
     PFB_KL();
     h->last_k = k;
-    if (out3k)
-        PFB_CK(cudaMemcpyAsync(out3k, h->d_out, sizeof(float) * 3 * (size_t)k,
-                               cudaMemcpyDeviceToHost, h->stream));
-    if (caer_k)
-        PFB_CK(cudaMemcpyAsync(caer_k, h->d_outc, sizeof(float) * (size_t)k,
-                               cudaMemcpyDeviceToHost, h->stream));
-    if (idx_k)
-        PFB_CK(cudaMemcpyAsync(idx_k, h->d_outi, sizeof(int) * (size_t)k,
-                               cudaMemcpyDeviceToHost, h->stream));
+    if (!host) {
+        if (out3k)
+            PFB_CK(cudaMemcpyAsync(out3k, h->d_out, sizeof(float) * 3 * (size_t)k,
+                                   cudaMemcpyDeviceToHost, h->stream));
+        if (caer_k)
+            PFB_CK(cudaMemcpyAsync(caer_k, h->d_outc, sizeof(float) * (size_t)k,
+                                   cudaMemcpyDeviceToHost, h->stream));
+        if (idx_k)
+            PFB_CK(cudaMemcpyAsync(idx_k, h->d_outi, sizeof(int) * (size_t)k,
+                                   cudaMemcpyDeviceToHost, h->stream));
+    }
     PFB_CK(cudaStreamSynchronize(h->stream));
+    if (host) {
+        if (out3k) memcpy(out3k, host->pose, sizeof(float) * 3 * (size_t)k);
+        if (caer_k) memcpy(caer_k, host->caer, sizeof(float) * (size_t)k);
+        if (idx_k) memcpy(idx_k, host->idx, sizeof(int) * (size_t)k);
+    }
     return k;
 }
 
@@ -1145,7 +1160,7 @@ int gl_localize_batch_enqueue(GlHandle* h, int nq, int per_q, int nrays, float r
 
 int gl_gather_topk(GlHandle* h, const uint64_t* sorted, int k) {
     k_gather_topk<<<ceil_div(k, kThreads), kThreads, 0, h->stream>>>(
-        sorted, k, h->d_hyp, h->d_caer, h->d_out, h->d_outc, h->d_outi);
+        sorted, k, h->d_hyp, h->d_caer, h->d_out, h->d_outc, h->d_outi, nullptr);
     PFB_KL();
     h->last_k = k;
     return 0;
@@ -1291,7 +1306,8 @@ void* pfgl_create(int W, int H, float res, float ox, float oy,
             break;
         if (cudaMalloc((void**)&h->d_ctl, sizeof(GlCtl)) != cudaSuccess) break;
         if (cudaMemset(h->d_ctl, 0, sizeof(GlCtl)) != cudaSuccess) break;
-        if (cudaMallocHost((void**)&h->h_ctl, sizeof(GlCtl)) != cudaSuccess)
+        if (cudaMallocHost((void**)&h->h_ctl, sizeof(GlCtl)) != cudaSuccess ||
+            cudaMallocHost((void**)&h->h_top, sizeof(TopHost)) != cudaSuccess)
             break;
         ok = true;
     } while (0);
@@ -1324,6 +1340,7 @@ int pfgl_destroy(void* hv) {
     cudaFree(h->d_sel);
     cudaFree(h->d_ctl);
     cudaFreeHost(h->h_ctl);
+    cudaFreeHost(h->h_top);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return 0;

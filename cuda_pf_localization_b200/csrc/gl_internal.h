@@ -27,6 +27,13 @@ struct GlCtl {
     unsigned long long visits;  // DDA cell visits counted by pfgl_count_visits
 };
 
+// The bottom-k a call returns, when it has at most kTop entries.
+struct TopHost {
+    static constexpr int kTop = 1024;
+    float pose[3 * kTop], caer[kTop];
+    int idx[kTop];
+};
+
 struct GlHandle {
     int dev = 0;
     int sms = 148;
@@ -55,6 +62,7 @@ struct GlHandle {
     uint64_t* d_sel = nullptr;   // small bottom-k select: the k smallest keys
     GlCtl* d_ctl = nullptr;
     GlCtl* h_ctl = nullptr;
+    TopHost* h_top = nullptr;  // pinned, written by k_gather_topk
     std::vector<unsigned char> host_grid;  // unpadded 0/1 copy
     bool caer_valid = false;
     int last_k = 0;  // entries of d_out written by the last bottom-k
