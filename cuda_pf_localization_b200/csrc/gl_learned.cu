@@ -1220,6 +1220,8 @@ struct LpHandle {
     // static parameters
     uint32_t* d_query = nullptr;
     float* h_res = nullptr;  // 3 kSelKMax poses, kSelKMax CAERs, kSelKMax indices
+    float* h_entries = nullptr;  // pinned: a batch of queries' bottom-k (pose, CAER, index)
+    size_t host_entries = 0;
     cudaGraph_t q_graph = nullptr;
     cudaGraphExec_t q_exec = nullptr;
     int q_n = 0, q_k = 0, q_nrays = 0;
@@ -1408,6 +1410,7 @@ void free_lp(LpHandle* h) {
     drop_query_graph(h);
     cudaFree(h->d_query);
     if (h->h_res) cudaFreeHost(h->h_res);
+    if (h->h_entries) cudaFreeHost(h->h_entries);
     for (int l = 0; l < kLayers; ++l) {
         Layer& L = h->L[l];
         cudaFree(L.w);
@@ -1619,19 +1622,29 @@ int learned_localize_batch(LpHandle* h, const float* scans, int nq, int nrays, f
                   "limits", n_samples, k);
         return -1;
     }
-    std::vector<float> o1(3 * (size_t)chunk * k), c1((size_t)chunk * k);
-    std::vector<int> i1((size_t)chunk * k);
+    // pinned: 1000 queries x 64 entries took 220 us longer through pageable memory
+    const size_t entries = (size_t)chunk * k;
+    if (entries > h->host_entries) {
+        cudaFreeHost(h->h_entries);
+        h->h_entries = nullptr;
+        h->host_entries = 0;
+        PFB_CK(cudaMallocHost((void**)&h->h_entries, 5 * sizeof(float) * entries));
+        h->host_entries = entries;
+    }
+    float* const o1 = h->h_entries;
+    float* const c1 = o1 + 3 * entries;
+    int* const i1 = reinterpret_cast<int*>(c1 + entries);
     for (int q0 = 0; q0 < nq; q0 += chunk) {
         const int m = std::min(chunk, nq - q0);
         const uint32_t qc0 = h->query_count;
         if (gl_upload_scans(g, scans + (size_t)q0 * nrays, m, nrays)) return -1;
         if (learned_batch_enqueue(h, m, nrays, rmax, span, n_samples, k)) return -1;
         const size_t mk = (size_t)m * k;
-        PFB_CK(cudaMemcpyAsync(o1.data(), g->d_out, sizeof(float) * 3 * mk,
+        PFB_CK(cudaMemcpyAsync(o1, g->d_out, sizeof(float) * 3 * mk,
                                cudaMemcpyDeviceToHost, h->stream));
-        PFB_CK(cudaMemcpyAsync(c1.data(), g->d_outc, sizeof(float) * mk,
+        PFB_CK(cudaMemcpyAsync(c1, g->d_outc, sizeof(float) * mk,
                                cudaMemcpyDeviceToHost, h->stream));
-        PFB_CK(cudaMemcpyAsync(i1.data(), g->d_outi, sizeof(int) * mk,
+        PFB_CK(cudaMemcpyAsync(i1, g->d_outi, sizeof(int) * mk,
                                cudaMemcpyDeviceToHost, h->stream));
         if (check_err(h)) return -1;  // synchronises
         for (int q = 0; q < m; ++q) {
@@ -1639,9 +1652,9 @@ int learned_localize_batch(LpHandle* h, const float* scans, int nq, int nrays, f
             const float best = c1[l];
             if (best_out) best_out[q0 + q] = best;
             int which = 0;
-            const float* os = o1.data() + 3 * l;
-            const float* cs = c1.data() + l;
-            const int* is = i1.data() + l;
+            const float* os = o1 + 3 * l;
+            const float* cs = c1 + l;
+            const int* is = i1 + l;
             std::vector<float> c2, o2;
             std::vector<int> i2;
             if (n_fallback > 0 && !(best <= tau)) {
