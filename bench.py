@@ -250,12 +250,14 @@ def reference_arm(args, world):
 
 # ------------------------------------------------------------ our GPU arm
 
-FP32_OPS_PER_PAIR = 29  # gated Cartesian term with the reference's roundings
-# DRAM bytes (read + write) of one k_weight launch at N = 1M, 256 observations,
-# from ncu (dram__bytes_read.sum + dram__bytes_write.sum; the capture command
-# is in profiles/pf_cycle_1M_scale.md): the poses are read from HBM, the
+# Rounded FP32 operations of the gated Cartesian weighting: a landmark moved into a
+# particle's frame (once, however often it is observed), and an observation against it.
+FP32_OPS_PER_MARK, FP32_OPS_PER_PAIR = 21, 8
+# DRAM bytes (read + write) of one weighting launch at N = 1M, 64 landmarks and 256
+# observations, from ncu (dram__bytes_read.sum + dram__bytes_write.sum; the capture
+# command is in profiles/pf_cycle_1M_scale.md): the poses are read from HBM, the
 # predicted poses and log-likelihoods it writes stay in L2.
-KWEIGHT_DRAM_BYTES_1M = 28.06e6
+WEIGHT_DRAM_BYTES_1M = 28.06e6
 # Algorithmic bytes per particle of each kernel of a resampling cycle, by the
 # library's kernel kinds: weight (fused predict + weighting: pose R 28 + W 28,
 # ll W 4), est (weight pass: ll R 4, w W 4), scan (run starts: w R 4), gather
@@ -794,39 +796,40 @@ def run_batched(args, torch, dev):
         mean_track_err_m=float(np.mean(errs)), n_min=int(sizes.min()), n_max=int(sizes.max()))
 
 
-def rooflines(val, n, nobs, t_cycle_s, hbm, peak_kind):
-    """The dominant kernel's roofline (k_weight: FP32 issue bound) and the
+def rooflines(val, n, marks, nobs, t_cycle_s, hbm, peak_kind):
+    """The dominant kernel's roofline (the weighting: FP32 issue bound) and the
     cycle's per-stage roofline sum_s max(B_s / BW, I_s / issue) / t_cycle."""
     ms, cnt = val["kernel_ms"], val["kernel_count"]
     per = {k: (ms[i] / cnt[i] if cnt[i] else 0.0) for i, k in enumerate(KINDS)}
     sm_mhz = val["clocks"]["sm_mhz"] or 1965.0
     issue_peak = 148 * 128 * sm_mhz * 1e6  # FP32 lane operations / s
     w_ms = per["weight"]
-    pair_rate = n * nobs / (w_ms * 1e-3)
-    achieved_ops = FP32_OPS_PER_PAIR * pair_rate
+    ops = n * (FP32_OPS_PER_MARK * min(marks, nobs) + FP32_OPS_PER_PAIR * nobs)
+    achieved_ops = ops / (w_ms * 1e-3)
     hbm_bytes = STAGE_BYTES["weight"] * n
-    roof = {"bound": "fp32 issue", "kernel": "k_weight (fused predict + gated weighting)",
+    roof = {"bound": "fp32 issue", "kernel": "k_weight_marks or k_weight (fused predict + gated weighting)",
             "achieved": achieved_ops / 1e12, "peak": issue_peak / 1e12,
             "unit": "T FP32 lane-ops/s", "frac": achieved_ops / issue_peak,
-            "traffic": (KWEIGHT_DRAM_BYTES_1M if (n, nobs) == (1_000_000, 256) else None),
-            "traffic_source": "ncu capture of one k_weight launch at this workload "
+            "traffic": (WEIGHT_DRAM_BYTES_1M if (n, marks, nobs) == (1_000_000, 64, 256) else None),
+            "traffic_source": "ncu capture of one weighting launch at this workload "
                               "(dram__bytes_read.sum + dram__bytes_write.sum)",
-            "ops_per_launch": FP32_OPS_PER_PAIR * n * nobs,
-            "ops_note": f"{FP32_OPS_PER_PAIR} rounded FP32 operations per particle-observation "
-                        "pair are required for the reference's bits (an FMA counts once); "
-                        "peak = 148 SM x 128 lanes x sampled SM clock",
+            "ops_per_launch": ops,
+            "ops_note": f"{FP32_OPS_PER_MARK} rounded FP32 operations per particle and landmark "
+                        f"and {FP32_OPS_PER_PAIR} per particle-observation pair are required for "
+                        "the reference's bits (an FMA counts once); the predict's are not "
+                        "counted; peak = 148 SM x 128 lanes x sampled SM clock",
             "avg_launch_ms": w_ms, "sm_mhz": sm_mhz,
             "hbm": {"achieved": hbm_bytes / (w_ms * 1e-3) / 1e9, "peak": hbm,
                     "unit": "GB/s", "frac": hbm_bytes / (w_ms * 1e-3) / 1e9 / hbm,
                     "alg_bytes_per_launch": hbm_bytes, "peak_source": peak_kind},
-            "timing": f"CUDA events around each k_weight launch on the library stream over "
+            "timing": f"CUDA events around each weighting launch on the library stream over "
                       f"the {val['profiled_steps']} cycles that continue the timed "
                       f"(graph-launched) cycles' trajectory (direct launches)"}
     stages = {}
     t_roof = 0.0
     for name, b in STAGE_BYTES.items():
         t_b = b * n / (hbm * 1e9)
-        t_i = (FP32_OPS_PER_PAIR * n * nobs / issue_peak) if name == "weight" else 0.0
+        t_i = ops / issue_peak if name == "weight" else 0.0
         t_s = max(t_b, t_i)
         t_roof += t_s
         stages[name] = {"alg_bytes_per_particle": b, "roof_us": 1e6 * t_s,
@@ -881,7 +884,7 @@ def main():
     e2e_value = multi.weak_scaling_rate(world, n * K, t_e2e)
     nobs = 256
     hbm, peak_kind = peaks()
-    roof, cycle_roof = rooflines(val, n, nobs, t_value / K, hbm, peak_kind)
+    roof, cycle_roof = rooflines(val, n, len(sc.landmarks), nobs, t_value / K, hbm, peak_kind)
     kernel_share = {name: float(val["kernel_ms"][i]) for i, name in enumerate(KINDS)}
     tot_k = sum(kernel_share.values())
 

@@ -1306,9 +1306,12 @@ void* pfgl_create(int W, int H, float res, float ox, float oy,
             break;
         if (cudaMalloc((void**)&h->d_ctl, sizeof(GlCtl)) != cudaSuccess) break;
         if (cudaMemset(h->d_ctl, 0, sizeof(GlCtl)) != cudaSuccess) break;
-        if (cudaMallocHost((void**)&h->h_ctl, sizeof(GlCtl)) != cudaSuccess ||
-            cudaMallocHost((void**)&h->h_top, sizeof(TopHost)) != cudaSuccess)
+        if (cudaMallocHost((void**)&h->h_ctl, sizeof(GlCtl)) != cudaSuccess)
             break;
+        if (cudaMallocHost((void**)&h->h_top, sizeof(TopHost)) != cudaSuccess) {
+            h->h_top = nullptr;  // the bottom-k is then copied
+            (void)cudaGetLastError();
+        }
         ok = true;
     } while (0);
     if (!ok) {

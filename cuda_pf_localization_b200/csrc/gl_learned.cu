@@ -1622,16 +1622,11 @@ int learned_localize_batch(LpHandle* h, const float* scans, int nq, int nrays, f
                   "limits", n_samples, k);
         return -1;
     }
-    // pinned: 1000 queries x 64 entries took 220 us longer through pageable memory
+    // through pinned memory when it holds a chunk: 1000 queries x 64 entries took 220 us
+    // longer through pageable memory
     const size_t entries = (size_t)chunk * k;
-    if (entries > h->host_entries) {
-        cudaFreeHost(h->h_entries);
-        h->h_entries = nullptr;
-        h->host_entries = 0;
-        PFB_CK(cudaMallocHost((void**)&h->h_entries, 5 * sizeof(float) * entries));
-        h->host_entries = entries;
-    }
-    float* const o1 = h->h_entries;
+    std::vector<float> pageable(entries > h->host_entries ? 5 * entries : 0);
+    float* const o1 = pageable.empty() ? h->h_entries : pageable.data();
     float* const c1 = o1 + 3 * entries;
     int* const i1 = reinterpret_cast<int*>(c1 + entries);
     for (int q0 = 0; q0 < nq; q0 += chunk) {
@@ -1768,6 +1763,13 @@ void* pfgl_learned_create(void* glv, int batch, unsigned long long seed) {
         if (make_mat(&h->tm_Xp, h->Xp, batch, kIn) ||
             make_mat(&h->tm_XpT, h->XpT, kIn, batch))
             break;
+        h->host_entries = (size_t)std::min(batch, 1024) * 64;
+        if (cudaMallocHost((void**)&h->h_entries, sizeof(float) * 5 * h->host_entries) !=
+            cudaSuccess) {
+            h->h_entries = nullptr;  // batches then go through pageable memory
+            h->host_entries = 0;
+            (void)cudaGetLastError();
+        }
         if (cudaMemsetAsync(h->Xp, 0, sizeof(bf16) * (size_t)batch * kIn,
                             h->stream) != cudaSuccess ||
             cudaMemsetAsync(h->d_err, 0, sizeof(unsigned), h->stream) != cudaSuccess)
