@@ -69,7 +69,7 @@ constexpr int BM = 128, BK = 64;
 // Output tile 128 x BN (BN = 128 or 256; the widest tcgen05 shape of one CTA
 // is 128 x 256).  Per k-block of 64 a 128 x 256 tile moves 48 KiB of
 // operands for 4.2 MFLOP, against 32 KiB for 2.1 MFLOP at 128 x 128: the
-// wider tile needs 30 % fewer operand bytes per flop from L2.
+// wider tile needs 25 % fewer operand bytes per flop from L2.
 constexpr uint32_t kWaitLimit = 1u << 24;
 
 enum Epi : int {

@@ -8,9 +8,9 @@
 //                 cloud first).
 //   pfc_weight    fused predict + weight + softmax partials, then the estimate
 //                 pass, the device Markley mean and the covariance pass around
-//                 that mean are queued speculatively, followed by one copy of
-//                 the control block to pinned host memory.
-//   pfc_est_sums  waits for that copy.
+//                 that mean are queued speculatively, the last kernel leaving
+//                 the control block in pinned host memory.
+//   pfc_est_sums  waits for that kernel.
 //   pfc_covs      returns the speculative covariances when the caller's f32
 //                 means equal the ones the device used (the Rust caller passes
 //                 exactly (float) of the returned sums and of its Markley
@@ -197,7 +197,7 @@ int device_error(PfHandle* h) {
 }
 
 // Queue estimate pass 1 + Markley (unless a fused resample already did) +
-// speculative covariance pass + the copy of the control block.
+// speculative covariance pass, which leaves the control block in host memory.
 // sq_from_ess: queued right after the weight pass (k_ess), whose sum w^2 the
 // estimate reports; skip_ratio: the caller's resampling rule (ess hint).
 int queue_estimate(PfHandle* h, bool sums_done = false, double skip_ratio = 0.0,

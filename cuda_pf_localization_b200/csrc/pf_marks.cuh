@@ -4,8 +4,9 @@
 // An observation's residual is the landmark in the particle's frame minus the
 // observed vector.  The landmark in the particle's frame (21 of the 29 f32
 // operations of a term) is the same for every observation of that landmark, so a
-// warp rotates its particles' landmarks once, keeps them on chip and takes the observations in their order against them: the operations and the
-// order of weight_two, to the bit.
+// warp rotates its particles' landmarks once, keeps them on chip and takes the
+// observations in their order against them: the operations and the order of
+// weight_two, to the bit.
 //
 // 24 bytes a landmark and lane (two particles) leave room for few warps, so the
 // loop lives on independent terms as much as on warps: kMBatch observations at a
@@ -15,7 +16,7 @@
 // memory.  Four further warps a group (scouts) predict the next tile's particles
 // and form the last one's softmax partial.
 //
-// 1M particles, 64 landmarks, 256 observations: 194 us against k_weight's 283; the
+// 1M particles, 64 landmarks, 256 observations: 188 us against k_weight's 286; the
 // f32 pipe is busy 60 % of the time, shared memory 50 %, the issue slots 60 % (the
 // 13.3 operations a pair that are left would take 91 us).  With one group (shared
 // memory, a warp a scheduler) 284: its latencies show.  One scout a group 217 and,

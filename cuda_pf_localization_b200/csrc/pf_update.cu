@@ -428,9 +428,9 @@ int launch_marks(PfHandle* h, const PredictArgs& pa, const CObservation* d_obs, 
 // Rotating a landmark once saves 21 of an observation's 29 operations for all but
 // its first, and costs a block the set-up and two tiles' latency.  k_weight and
 // k_weight_marks measured (us, particles x landmarks / observations): 1M x 64/256
-// 283 and 194, 1M x 12/128 160 and 109, 1M x 32/96 131 and 113, 1M x 32/64 100 and
-// 100, 200k x 32/128 45 and 41, 100k x 64/256 45 and 43, 100k x 64/192 38 and 39,
-// 200k x 64/128 45 and 47.
+// 286 and 188, 1M x 12/128 161 and 100, 1M x 32/96 129 and 104, 1M x 32/64 98 and
+// 91, 200k x 32/128 44 and 39, 100k x 64/256 44 and 38, 100k x 64/192 36 and 34,
+// 200k x 64/128 44 and 45.
 bool weight_by_marks(const PfHandle* h, int nobs, bool cart) {
     return cart && h->weight_variant == 0 && h->lm_count > 0 && h->lm_count <= kMMarks &&
            nobs <= kMObs && nobs >= 96 && nobs >= 2 * h->lm_count &&
