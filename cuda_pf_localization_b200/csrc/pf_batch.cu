@@ -219,6 +219,7 @@ __global__ void __launch_bounds__(kWThreads, 6)
     const int nobs = in.nobs;
     if (nobs <= 0) {
         // predict only: the single-filter cycle resets the weights to uniform
+        __syncthreads();  // the whole tile has read the generation
         if (threadIdx.x == 0 && atomicAdd(&c->done_w, 1u) == (unsigned)fl.nwtiles - 1u) {
             c->wmode = WMODE_UNIFORM;
             c->gen = pa.gen;
