@@ -261,8 +261,13 @@ bool all_cartesian(const CObservation* obs, int nobs) {
 
 bool valid_handle(PfHandle* h) { return h != nullptr && h->n > 0; }
 
-// Everything a captured cycle depends on besides the per-cycle values.
-void cycle_graph_key(const PfHandle* h, const PfcCycleParams* prm, long long k[12]) {
+// Everything a captured cycle depends on besides the per-cycle values.  The injection
+// buckets are freed and allocated anew when a larger ratio (of a cycle that replays the
+// other graph, or of a resample between two cycles) needs more room, so a graph that
+// uses them holds for one allocation and its room per tile only: a freed address may
+// come back with another size.
+void cycle_graph_key(const PfHandle* h, const PfcCycleParams* prm, int kinj,
+                     long long (&k)[PfHandle::kGraphKey]) {
     auto f2l = [](float v) { long long r = 0; memcpy(&r, &v, sizeof v); return r; };
     long long e = 0;
     memcpy(&e, &prm->resample_ess_ratio, sizeof e);
@@ -277,7 +282,8 @@ void cycle_graph_key(const PfHandle* h, const PfcCycleParams* prm, long long k[1
     k[8] = f2l(prm->random_inject_ratio);
     k[9] = h->weight_variant;
     k[10] = h->record_anc ? 1 : 0;
-    k[11] = 1;
+    k[11] = kinj > 0 ? (long long)(uintptr_t)h->d_inj_bucket : 0;
+    k[12] = kinj > 0 ? h->inj_cap : 0;
 }
 
 int enqueue_cycle(PfHandle* h, const PredictArgs& pa, const CObservation* obs_dev,
@@ -314,8 +320,8 @@ int run_cycle_graph(PfHandle* h, const PfcOdom* odom, const CObservation* obs_de
                            h->stream));
     PFB_CK(cudaEventRecord(h->cargs_ev[slot], h->stream));
     h->stats.h2d_bytes += sizeof(CycleArgs);
-    long long key[12];
-    cycle_graph_key(h, prm, key);
+    long long key[PfHandle::kGraphKey];
+    cycle_graph_key(h, prm, kinj, key);
     PfHandle::CycleGraph& cg = h->cyc[weight_by_marks(h, nobs, cart) ? 1 : 0];
     if (cg.exec && memcmp(key, cg.key, sizeof key) != 0) drop_cycle_graph(cg);
     if (!cg.exec) {
@@ -335,6 +341,7 @@ int run_cycle_graph(PfHandle* h, const PfcOdom* odom, const CObservation* obs_de
         }
         cg.graph = g;
         PFB_CK(cudaGraphInstantiate(&cg.exec, g, 0));
+        h->graph_captures += 1;
         memcpy(cg.key, key, sizeof key);
     }
     PFB_CK(cudaGraphLaunch(cg.exec, h->stream));
@@ -809,6 +816,11 @@ int pfc_set_graph(void* hv, int on) {
     h->use_graph = on != 0;
     if (!h->use_graph) drop_cycle_graphs(h);
     return 0;
+}
+
+long long pfc_graph_captures(void* hv) {
+    PfHandle* h = as_pf(hv);
+    return h ? h->graph_captures : -1;
 }
 
 int pfc_cycle_result(void* hv, double* est_out) {

@@ -292,12 +292,14 @@ struct PfHandle {
     bool use_graph = true;
     // one for each weighting kernel, so a change of the observation count that
     // changes the kernel does not capture again
+    static constexpr int kGraphKey = 13;
     struct CycleGraph {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
-        long long key[12] = {};
+        long long key[kGraphKey] = {};
         int kernels = 0;
     } cyc[2];
+    long long graph_captures = 0;  // of both, so far
 
     // accounting: kernels launched, bytes copied host<->device, host syncs
     PfcStats stats{};

@@ -200,10 +200,14 @@ int pfc_cycle_result(void* h, double* est_out);
 
 /* 1 (default): a fused cycle with observations is replayed from a CUDA graph
  * captured on first use (re-captured when n, the landmark table, the cycle
- * parameters or the weighting variant change); 0: direct kernel launches.
+ * parameters, the injection's buffers or the weighting variant change); 0:
+ * direct kernel launches.
  * Both give identical results.  Cycles run with per-kernel profiling
  * (pfc_profile) always use direct launches. */
 int pfc_set_graph(void* h, int on);
+/* Cycle graphs captured by this handle so far (a test hook: a graph whose
+ * buffers have been replaced has to be captured again); -1 without a handle. */
+long long pfc_graph_captures(void* h);
 
 /* Sharded filter (no counterpart in the reference): one filter of n
  * particles over `world` ranks (one handle per rank, normally one GPU each).
