@@ -1220,8 +1220,6 @@ struct LpHandle {
     // static parameters
     uint32_t* d_query = nullptr;
     float* h_res = nullptr;  // 3 kSelKMax poses, kSelKMax CAERs, kSelKMax indices
-    float* h_entries = nullptr;  // pinned: a batch of queries' bottom-k (pose, CAER, index)
-    size_t host_entries = 0;
     cudaGraph_t q_graph = nullptr;
     cudaGraphExec_t q_exec = nullptr;
     int q_n = 0, q_k = 0, q_nrays = 0;
@@ -1410,7 +1408,6 @@ void free_lp(LpHandle* h) {
     drop_query_graph(h);
     cudaFree(h->d_query);
     if (h->h_res) cudaFreeHost(h->h_res);
-    if (h->h_entries) cudaFreeHost(h->h_entries);
     for (int l = 0; l < kLayers; ++l) {
         Layer& L = h->L[l];
         cudaFree(L.w);
@@ -1622,42 +1619,36 @@ int learned_localize_batch(LpHandle* h, const float* scans, int nq, int nrays, f
                   "limits", n_samples, k);
         return -1;
     }
-    // through pinned memory when it holds a chunk: 1000 queries x 64 entries took 220 us
-    // longer through pageable memory
-    const size_t entries = (size_t)chunk * k;
-    std::vector<float> pageable(entries > h->host_entries ? 5 * entries : 0);
-    float* const o1 = pageable.empty() ? h->h_entries : pageable.data();
-    float* const c1 = o1 + 3 * entries;
-    int* const i1 = reinterpret_cast<int*>(c1 + entries);
+    // The results are copied to where the caller wants them; the CAERs are read here.
+    // (Through vectors, allocated and cleared on each call, 1000 queries of 64 entries
+    // took 220 us longer.)
+    std::vector<float> caer_tmp(caer_k ? 0 : (size_t)chunk * k);
     for (int q0 = 0; q0 < nq; q0 += chunk) {
         const int m = std::min(chunk, nq - q0);
         const uint32_t qc0 = h->query_count;
         if (gl_upload_scans(g, scans + (size_t)q0 * nrays, m, nrays)) return -1;
         if (learned_batch_enqueue(h, m, nrays, rmax, span, n_samples, k)) return -1;
-        const size_t mk = (size_t)m * k;
-        PFB_CK(cudaMemcpyAsync(o1, g->d_out, sizeof(float) * 3 * mk,
-                               cudaMemcpyDeviceToHost, h->stream));
-        PFB_CK(cudaMemcpyAsync(c1, g->d_outc, sizeof(float) * mk,
-                               cudaMemcpyDeviceToHost, h->stream));
-        PFB_CK(cudaMemcpyAsync(i1, g->d_outi, sizeof(int) * mk,
-                               cudaMemcpyDeviceToHost, h->stream));
+        const size_t mk = (size_t)m * k, at = (size_t)q0 * k;
+        float* const caers = caer_k ? caer_k + at : caer_tmp.data();
+        if (out3k)
+            PFB_CK(cudaMemcpyAsync(out3k + 3 * at, g->d_out, sizeof(float) * 3 * mk,
+                                   cudaMemcpyDeviceToHost, h->stream));
+        PFB_CK(cudaMemcpyAsync(caers, g->d_outc, sizeof(float) * mk, cudaMemcpyDeviceToHost,
+                               h->stream));
+        if (idx_k)
+            PFB_CK(cudaMemcpyAsync(idx_k + at, g->d_outi, sizeof(int) * mk,
+                                   cudaMemcpyDeviceToHost, h->stream));
         if (check_err(h)) return -1;  // synchronises
         for (int q = 0; q < m; ++q) {
-            const size_t o = (size_t)(q0 + q) * k, l = (size_t)q * k;
-            const float best = c1[l];
+            const size_t o = at + (size_t)q * k;
+            const float best = caers[(size_t)q * k];
             if (best_out) best_out[q0 + q] = best;
             int which = 0;
-            const float* os = o1 + 3 * l;
-            const float* cs = c1 + l;
-            const int* is = i1 + l;
-            std::vector<float> c2, o2;
-            std::vector<int> i2;
             if (n_fallback > 0 && !(best <= tau)) {
                 const int n_pos = std::max(1, n_fallback / 16);
                 const int kk = std::min(k, n_pos * 16);
-                c2.assign(k, INFINITY);
-                o2.assign(3 * (size_t)k, 0.f);
-                i2.assign(k, -1);
+                std::vector<float> c2(k, INFINITY), o2(3 * (size_t)k, 0.f);
+                std::vector<int> i2(k, -1);
                 if (gl_upload_scan(g, scans + (size_t)(q0 + q) * nrays, nrays) ||
                     gl_generate(g, n_pos, 16,
                                 h->seed + 0x9E3779B97F4A7C15ULL * (qc0 + (uint64_t)q + 1)))
@@ -1668,14 +1659,11 @@ int learned_localize_batch(LpHandle* h, const float* scans, int nq, int nrays, f
                 which = 1;
                 if (c2[0] < best) {
                     which = 2;
-                    os = o2.data();
-                    cs = c2.data();
-                    is = i2.data();
+                    if (out3k) memcpy(out3k + 3 * o, o2.data(), sizeof(float) * 3 * (size_t)k);
+                    if (caer_k) memcpy(caer_k + o, c2.data(), sizeof(float) * (size_t)k);
+                    if (idx_k) memcpy(idx_k + o, i2.data(), sizeof(int) * (size_t)k);
                 }
             }
-            if (out3k) memcpy(out3k + 3 * o, os, sizeof(float) * 3 * (size_t)k);
-            if (caer_k) memcpy(caer_k + o, cs, sizeof(float) * (size_t)k);
-            if (idx_k) memcpy(idx_k + o, is, sizeof(int) * (size_t)k);
             if (info) info[q0 + q] = which;
         }
     }
@@ -1763,13 +1751,6 @@ void* pfgl_learned_create(void* glv, int batch, unsigned long long seed) {
         if (make_mat(&h->tm_Xp, h->Xp, batch, kIn) ||
             make_mat(&h->tm_XpT, h->XpT, kIn, batch))
             break;
-        h->host_entries = (size_t)std::min(batch, 1024) * 64;
-        if (cudaMallocHost((void**)&h->h_entries, sizeof(float) * 5 * h->host_entries) !=
-            cudaSuccess) {
-            h->h_entries = nullptr;  // batches then go through pageable memory
-            h->host_entries = 0;
-            (void)cudaGetLastError();
-        }
         if (cudaMemsetAsync(h->Xp, 0, sizeof(bf16) * (size_t)batch * kIn,
                             h->stream) != cudaSuccess ||
             cudaMemsetAsync(h->d_err, 0, sizeof(unsigned), h->stream) != cudaSuccess)
