@@ -1306,12 +1306,9 @@ void* pfgl_create(int W, int H, float res, float ox, float oy,
             break;
         if (cudaMalloc((void**)&h->d_ctl, sizeof(GlCtl)) != cudaSuccess) break;
         if (cudaMemset(h->d_ctl, 0, sizeof(GlCtl)) != cudaSuccess) break;
-        if (cudaMallocHost((void**)&h->h_ctl, sizeof(GlCtl)) != cudaSuccess)
+        if (cudaMallocHost((void**)&h->h_ctl, sizeof(GlCtl) + sizeof(TopHost)) != cudaSuccess)
             break;
-        if (cudaMallocHost((void**)&h->h_top, sizeof(TopHost)) != cudaSuccess) {
-            h->h_top = nullptr;  // the bottom-k is then copied
-            (void)cudaGetLastError();
-        }
+        h->h_top = reinterpret_cast<TopHost*>(h->h_ctl + 1);
         ok = true;
     } while (0);
     if (!ok) {
@@ -1343,7 +1340,6 @@ int pfgl_destroy(void* hv) {
     cudaFree(h->d_sel);
     cudaFree(h->d_ctl);
     cudaFreeHost(h->h_ctl);
-    cudaFreeHost(h->h_top);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return 0;

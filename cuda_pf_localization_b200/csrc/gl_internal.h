@@ -61,8 +61,8 @@ struct GlHandle {
     uint64_t* d_cand = nullptr;  // pruned-scorer survivors (cap_hyp)
     uint64_t* d_sel = nullptr;   // small bottom-k select: the k smallest keys
     GlCtl* d_ctl = nullptr;
-    GlCtl* h_ctl = nullptr;
-    TopHost* h_top = nullptr;  // pinned, written by k_gather_topk
+    GlCtl* h_ctl = nullptr;    // pinned, with h_top behind it in one allocation
+    TopHost* h_top = nullptr;  // written by k_gather_topk
     std::vector<unsigned char> host_grid;  // unpadded 0/1 copy
     bool caer_valid = false;
     int last_k = 0;  // entries of d_out written by the last bottom-k

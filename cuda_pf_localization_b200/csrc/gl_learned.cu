@@ -1219,7 +1219,10 @@ struct LpHandle {
     // the results copied to pinned memory, the graph keyed on the query's
     // static parameters
     uint32_t* d_query = nullptr;
-    float* h_res = nullptr;  // 3 kSelKMax poses, kSelKMax CAERs, kSelKMax indices
+    // pinned, one allocation (a millisecond or more each, whatever its size): 3 kSelKMax
+    // poses, kSelKMax CAERs, kSelKMax indices, then host_entries of the same of a batch
+    float* h_res = nullptr;
+    size_t host_entries = 0;
     cudaGraph_t q_graph = nullptr;
     cudaGraphExec_t q_exec = nullptr;
     int q_n = 0, q_k = 0, q_nrays = 0;
@@ -1619,26 +1622,38 @@ int learned_localize_batch(LpHandle* h, const float* scans, int nq, int nrays, f
                   "limits", n_samples, k);
         return -1;
     }
-    // The results are copied to where the caller wants them; the CAERs are read here.
-    // (Through vectors, allocated and cleared on each call, 1000 queries of 64 entries
-    // took 220 us longer.)
-    std::vector<float> caer_tmp(caer_k ? 0 : (size_t)chunk * k);
+    // The results come through pinned memory when it holds a chunk, else straight to
+    // where the caller wants them (1000 queries of 64 entries: 3.08 and 3.17 ms; through
+    // vectors, allocated and cleared on each call, 220 us longer than the first).
+    const size_t entries = (size_t)chunk * k;
+    float* const pinned = entries <= h->host_entries ? h->h_res + 5 * kSelKMax : nullptr;
+    std::vector<float> caer_tmp(pinned || caer_k ? 0 : entries);
     for (int q0 = 0; q0 < nq; q0 += chunk) {
         const int m = std::min(chunk, nq - q0);
         const uint32_t qc0 = h->query_count;
         if (gl_upload_scans(g, scans + (size_t)q0 * nrays, m, nrays)) return -1;
         if (learned_batch_enqueue(h, m, nrays, rmax, span, n_samples, k)) return -1;
         const size_t mk = (size_t)m * k, at = (size_t)q0 * k;
-        float* const caers = caer_k ? caer_k + at : caer_tmp.data();
-        if (out3k)
-            PFB_CK(cudaMemcpyAsync(out3k + 3 * at, g->d_out, sizeof(float) * 3 * mk,
+        float* const pose = out3k ? out3k + 3 * at : nullptr;
+        float* const caer = caer_k ? caer_k + at : nullptr;
+        int* const idx = idx_k ? idx_k + at : nullptr;
+        float* const from_pose = pinned ? pinned : pose;
+        float* const caers = pinned ? pinned + 3 * entries : caer ? caer : caer_tmp.data();
+        int* const from_idx = pinned ? reinterpret_cast<int*>(pinned + 4 * entries) : idx;
+        if (pose)
+            PFB_CK(cudaMemcpyAsync(from_pose, g->d_out, sizeof(float) * 3 * mk,
                                    cudaMemcpyDeviceToHost, h->stream));
         PFB_CK(cudaMemcpyAsync(caers, g->d_outc, sizeof(float) * mk, cudaMemcpyDeviceToHost,
                                h->stream));
-        if (idx_k)
-            PFB_CK(cudaMemcpyAsync(idx_k + at, g->d_outi, sizeof(int) * mk,
+        if (idx)
+            PFB_CK(cudaMemcpyAsync(from_idx, g->d_outi, sizeof(int) * mk,
                                    cudaMemcpyDeviceToHost, h->stream));
         if (check_err(h)) return -1;  // synchronises
+        if (pinned) {
+            if (pose) memcpy(pose, from_pose, sizeof(float) * 3 * mk);
+            if (caer) memcpy(caer, caers, sizeof(float) * mk);
+            if (idx) memcpy(idx, from_idx, sizeof(int) * mk);
+        }
         for (int q = 0; q < m; ++q) {
             const size_t o = at + (size_t)q * k;
             const float best = caers[(size_t)q * k];
@@ -1743,9 +1758,12 @@ void* pfgl_learned_create(void* glv, int batch, unsigned long long seed) {
             dalloc(&h->Yp, (size_t)batch * 4) || dalloc(&h->d_err, 1) ||
             dalloc(&h->d_best, 64) || dalloc(&h->d_query, 1))
             break;
-        if (cudaMallocHost((void**)&h->h_res, sizeof(float) * 5 * kSelKMax) !=
-            cudaSuccess) {
+        // 64 entries a query of a batch, of up to 1024
+        h->host_entries = (size_t)std::min(batch, 1024) * 64;
+        if (cudaMallocHost((void**)&h->h_res,
+                           sizeof(float) * 5 * (kSelKMax + h->host_entries)) != cudaSuccess) {
             h->h_res = nullptr;  // queries then use direct launches
+            h->host_entries = 0;
             (void)cudaGetLastError();
         }
         if (make_mat(&h->tm_Xp, h->Xp, batch, kIn) ||
