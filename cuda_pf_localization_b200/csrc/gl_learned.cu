@@ -125,7 +125,7 @@ __device__ __forceinline__ void epilogue_chunk(const uint32_t (&r)[32], uint32_t
         const float4* b4 = reinterpret_cast<const float4*>(ep.bias + col0);
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const float4 b = __ldg(&b4[q]);
+            const float4 b = b4[q];
             bias[4 * q] = b.x;
             bias[4 * q + 1] = b.y;
             bias[4 * q + 2] = b.z;
@@ -209,8 +209,8 @@ __device__ __forceinline__ void load_gates(uint32_t (&g)[kMine], int row0, int n
     if constexpr (EPI == EPI_DRELU_BF16) {
 #pragma unroll
         for (int i = 0; i < kMine; ++i)
-            g[i] = __ldg(&ep.bits[(size_t)((n0 >> 5) + part + i * kPerQ) * ep.ldb + row0 +
-                                  (threadIdx.x & 31)]);
+            g[i] = __ldcg(&ep.bits[(size_t)((n0 >> 5) + part + i * kPerQ) * ep.ldb + row0 +
+                                   (threadIdx.x & 31)]);
     }
 }
 
@@ -606,8 +606,8 @@ __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + expf
 // Gradients are scaled by inv_b (mean over the batch) and written as bf16
 // (padding columns 288..383 zero).
 __global__ void __launch_bounds__(256)
-    k_gmm_loss(const float* __restrict__ Z, const float* __restrict__ Y, int y_row0,
-               int rows, float inv_b, bf16* __restrict__ dZ, float* __restrict__ loss_acc) {
+    k_gmm_loss(const float* Z, const float* Y, int y_row0, int rows, float inv_b,
+               bf16* __restrict__ dZ, float* __restrict__ loss_acc) {
     __shared__ float s_loss[8];
     pdl_trigger();
     pdl_wait();
@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(256)
 // out[c][r] = in[r][c] for an R x C bf16 matrix, in 64 x 64 tiles through
 // shared memory; tile rows are read and written as bf16 pairs (4-byte
 // accesses, 128 bytes per warp) where the strides and base addresses allow.
-__global__ void k_transpose_bf16(const bf16* __restrict__ in, long long ld_in,
+__global__ void k_transpose_bf16(const bf16* in, long long ld_in,
                                  bf16* __restrict__ out, long long ld_out,
                                  long long R, long long C) {
     __shared__ bf16 t[64][66];

@@ -892,7 +892,7 @@ __global__ void k_b_inject_apply(Arena A, const BFilter* __restrict__ F,
 // them.  One block per filter; the others take the estimate pass.
 __global__ void __launch_bounds__(kThreads)
     k_b_est_src(const BFilter* __restrict__ F, BCtl* C, BGlobal* G,
-                const double* __restrict__ gpart, const double* __restrict__ icorr) {
+                const double* gpart, const double* icorr) {
     const BFilter& fl = F[blockIdx.x];
     BCtl* c = C + blockIdx.x;
     pdl_wait();

@@ -285,6 +285,10 @@ __host__ __device__ __forceinline__ long long ceil_div_ll(long long a,
 // return, so completion stays transitive along the chain (a kernel that ended
 // without waiting could finish before the kernel two back).  A no-op for a
 // plain launch.
+// What an earlier kernel of the chain writes is not constant for the lifetime of
+// such a kernel, so it is read by plain or L2 loads: no const __restrict__
+// parameter and no __ldg, which let the compiler take it for constant (the
+// non-coherent path, a load moved before the wait).
 __device__ __forceinline__ void pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -53,9 +53,8 @@ __device__ bool block_reduce_last(double (&acc)[NV], double* part,
 }
 
 __global__ void __launch_bounds__(kThreads, 2)
-    k_est_sums(PlaneSet ps, int n, const float* __restrict__ ll,
-               float* __restrict__ w, double* part, unsigned* done,
-               CycleCtl* ctl, int sq_from_ess, double skip_ratio) {
+    k_est_sums(PlaneSet ps, int n, const float* ll, float* __restrict__ w, double* part,
+               unsigned* done, CycleCtl* ctl, int sq_from_ess, double skip_ratio) {
     pdl_wait();
     if (sq_from_ess && skip_ratio > 0.0) {
         // the caller resamples when this estimate's ESS is below
@@ -145,9 +144,8 @@ __device__ __forceinline__ void control_to_host(const CycleCtl* ctl, CycleCtl* h
 // discards this estimate's covariances; the pass is skipped in that case and
 // the cached mean is made unusable, so pfc_covs computes them on demand.
 __global__ void __launch_bounds__(kThreads, 2)
-    k_covs(PlaneSet ps, int n, const float* __restrict__ ll,
-           const float* __restrict__ w, double* part, unsigned* done,
-           CycleCtl* ctl, int use_args, float3 mp_arg, float4 mq_arg,
+    k_covs(PlaneSet ps, int n, const float* ll, const float* w, double* part,
+           unsigned* done, CycleCtl* ctl, int use_args, float3 mp_arg, float4 mq_arg,
            int mode, double skip_ratio, CycleCtl* host) {
     pdl_wait();
     if (skip_ratio > 0.0 && ctl->ess < skip_ratio * (double)n) {
@@ -245,7 +243,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 // block, so the grid fills every SM; the FP64 sum is reduced in a fixed order
 // (block butterfly, then block partials in block order).
 __global__ void __launch_bounds__(kThreads)
-    k_ess(int n, const float* __restrict__ ll, float* __restrict__ w,
+    k_ess(int n, const float* ll, float* __restrict__ w,
           double* part, unsigned long long* partu, uint64_t* prefix,
           unsigned* done, CycleCtl* ctl, int decide, double ess_ratio) {
     pdl_wait();

@@ -183,11 +183,10 @@ __device__ __forceinline__ void apply_draws(const InjList& L, int m, int l0,
 // Each block leaves one partial of the 14 sums (the positions before the
 // injection); block 0 of k_gather combines them.
 __global__ void __launch_bounds__(kThreads, 2)
-    k_mark(PlaneBase pb, int n, const float* __restrict__ w, const float* __restrict__ ll,
-           const uint64_t* __restrict__ prefix, int* __restrict__ marker,
-           int* __restrict__ inj_cnt, int* __restrict__ inj_bucket, int inj_cap, int k_inj,
-           uint64_t gen, double* part_m, CycleCtl* ctl, int cond, int use_u01,
-           double u01_arg, const CycleArgs* ca) {
+    k_mark(PlaneBase pb, int n, const float* w, const float* ll, const uint64_t* prefix,
+           int* __restrict__ marker, int* __restrict__ inj_cnt, int* __restrict__ inj_bucket,
+           int inj_cap, int k_inj, uint64_t gen, double* part_m, CycleCtl* ctl, int cond,
+           int use_u01, double u01_arg, const CycleArgs* ca) {
     pdl_wait();
     if (ca) gen = ca->gen;
     const bool resample = !cond || ctl->resample_now;
@@ -352,7 +351,7 @@ struct GatherSmem {
 // position sums and commits the resample.
 __global__ void __launch_bounds__(kThreads, 4)
     k_gather(PlaneBase pb, int n, int* __restrict__ marker, int* __restrict__ anc,
-             int record, int* __restrict__ inj_cnt, const int* __restrict__ inj_bucket,
+             int record, int* __restrict__ inj_cnt, const int* inj_bucket,
              int inj_cap, int k_inj, uint64_t gen, const double* part_m, int mark_grid,
              double* part_c, unsigned* done, CycleCtl* ctl, int cond, int use_u01,
              double u01_arg, const CycleArgs* ca) {
