@@ -827,10 +827,10 @@ __global__ void k_b_inject_link(const BFilter* __restrict__ F, const BCtl* C,
                                 const BGlobal* G, const int* __restrict__ draw_f,
                                 int total, uint64_t* head, int* next) {
     const int d = blockIdx.x * kThreads + threadIdx.x;
+    pdl_wait();
     if (d >= total) return;
     const int f = draw_f[d];
     const BCtl& c = C[f];
-    pdl_wait();
     if (!c.resample_now || !c.resample_valid) return;
     const BFilter& fl = F[f];
     const InjDraw dr = inj_draw(c.lcg_next, c.gen, d - fl.inj_off, fl.n);
@@ -850,10 +850,10 @@ __global__ void k_b_inject_apply(Arena A, const BFilter* __restrict__ F,
                                  const uint64_t* head, const int* next,
                                  double* __restrict__ icorr) {
     const int d = blockIdx.x * kThreads + threadIdx.x;
+    pdl_wait();
     if (d >= total) return;
     const int f = draw_f[d];
     const BCtl& c = C[f];
-    pdl_wait();
     if (!c.resample_now || !c.resample_valid) return;
     const BFilter& fl = F[f];
     const uint64_t lcg = c.lcg_next;

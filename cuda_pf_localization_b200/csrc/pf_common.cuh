@@ -277,14 +277,16 @@ __host__ __device__ __forceinline__ long long ceil_div_ll(long long a,
 }
 
 // ------------------------------------------------- programmatic dependent launch
-// The kernels of a filter cycle and of a training step are launched with
-// programmatic stream serialisation: a kernel's blocks may be scheduled as soon as every block
-// of its predecessor has exited, before the predecessor grid is retired, and
-// wait at pdl_wait() until the predecessor grid has completed and its memory
-// is visible.  Every such kernel calls pdl_wait() first, before any early
-// return, so completion stays transitive along the chain (a kernel that ended
-// without waiting could finish before the kernel two back).  A no-op for a
-// plain launch.
+// The kernels of a filter cycle, of a batch's cycle and of a training step are
+// launched with programmatic stream serialisation: a kernel's blocks may be
+// scheduled as soon as every block of its predecessor has exited or called
+// pdl_trigger(), before the predecessor grid is retired, and wait at pdl_wait()
+// until the predecessor grid has completed and its memory is visible.  Every such
+// kernel calls pdl_wait() in all its threads and before any return, so no block ends
+// without waiting and completion stays transitive along the chain (a kernel that
+// ended without waiting could finish before the kernel two back).  Before the wait
+// come only reads of host-written tables and a block's own set-up (barriers, tensor
+// memory).  A no-op for a plain launch.
 // What an earlier kernel of the chain writes is not constant for the lifetime of
 // such a kernel, so it is read by plain or L2 loads: no const __restrict__
 // parameter and no __ldg, which let the compiler take it for constant (the

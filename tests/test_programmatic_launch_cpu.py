@@ -1,6 +1,7 @@
 """Rules of the kernels that are launched before their predecessor's end, checked in
-their source: a load that the compiler may take for constant must not read what an
-earlier kernel of the chain writes."""
+their source: no thread leaves before it has waited for the predecessor, and a load
+that the compiler may take for constant must not read what an earlier kernel of the
+chain writes."""
 import re
 from pathlib import Path
 
@@ -63,3 +64,10 @@ def test_constant_loads():
     for path in list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")):
         for arg in re.findall(r"__ldg\(\s*&((?:[^()]|\([^()]*\))*)\)", _source(path)):
             assert re.sub(r"\s+", "", arg) in CONSTANT_LOADS, (path.name, arg)
+
+
+@pytest.mark.parametrize("name,body", [(n, b) for n, _, b in KERNELS],
+                         ids=[n for n, _, _ in KERNELS])
+def test_no_thread_leaves_before_the_wait(name, body):
+    assert body.count("pdl_wait()") == 1
+    assert not re.search(r"\breturn\b", body[:body.index("pdl_wait()")])
