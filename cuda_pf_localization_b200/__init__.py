@@ -134,6 +134,7 @@ _KERNEL_SIGS = {
                                  POINTER(PfcCycleParams), _dp]),
     "pfc_cycle_result": (c_int, [c_void_p, _dp]),
     "pfc_set_graph": (c_int, [c_void_p, c_int]),
+    "pfc_set_wait_test": (c_int, [c_void_p, c_int]),
     "pfc_graph_captures": (C.c_longlong, [c_void_p]),
     "pfc_shard_init": (c_int, [c_void_p, c_int, c_int, c_int, c_uint]),
     "pfc_shard_layout": (c_int, [c_void_p, _ip, _ip]),

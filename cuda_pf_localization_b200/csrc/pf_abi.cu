@@ -284,6 +284,7 @@ void cycle_graph_key(const PfHandle* h, const PfcCycleParams* prm, int kinj,
     k[10] = h->record_anc ? 1 : 0;
     k[11] = kinj > 0 ? (long long)(uintptr_t)h->d_inj_bucket : 0;
     k[12] = kinj > 0 ? h->inj_cap : 0;
+    k[13] = h->wait_polls;
 }
 
 int enqueue_cycle(PfHandle* h, const PredictArgs& pa, const CObservation* obs_dev,
@@ -815,6 +816,16 @@ int pfc_set_graph(void* hv, int on) {
     if (!h) return -1;
     h->use_graph = on != 0;
     if (!h->use_graph) drop_cycle_graphs(h);
+    return 0;
+}
+
+int pfc_set_wait_test(void* hv, int polls) {
+    PfHandle* h = as_pf(hv);
+    if (!h || polls < -1) {
+        set_error("pf_b200: pfc_set_wait_test: polls %d", polls);
+        return -1;
+    }
+    h->wait_polls = polls < 0 ? PfHandle::kWaitPolls : (unsigned)polls;
     return 0;
 }
 

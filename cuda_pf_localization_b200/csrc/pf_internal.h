@@ -278,6 +278,8 @@ struct PfHandle {
     cudaEvent_t est_ev = nullptr;
 
     int weight_variant = 0;
+    static constexpr unsigned kWaitPolls = 1u << 24;
+    unsigned wait_polls = kWaitPolls;  // of a wait inside a weighting block
     bool record_anc = false;
     bool anc_valid = false;
     unsigned inj_epoch = 0;    // injection list epoch (never 0 when used)
@@ -292,7 +294,7 @@ struct PfHandle {
     bool use_graph = true;
     // one for each weighting kernel, so a change of the observation count that
     // changes the kernel does not capture again
-    static constexpr int kGraphKey = 13;
+    static constexpr int kGraphKey = 14;
     struct CycleGraph {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;

@@ -44,7 +44,6 @@ constexpr int kMThreads = 32 * kMGroups * (kMMarkers + kMScouts);
 constexpr int kMBatch = 4;
 constexpr int kMColumns = 8;    // tensor-memory columns of a landmark (six used)
 constexpr int kMSlotBytes = 3 * 32 * (int)sizeof(float2);  // shared memory of a landmark
-constexpr unsigned kMWaitLimit = 1u << 24;
 static_assert(kMTile == 2 * kWThreads, "a group takes a softmax tile");
 static_assert(kMThreads >= kMObs, "an observation a thread in marks_build");
 static_assert(kMMarks * kMColumns == 512, "all columns of tensor memory");
@@ -67,10 +66,11 @@ struct MarksSmem {
     uint32_t tmem;
 };
 
-// Wait of a whole warp for a phase of one of the block's barriers; false when it
-// or another of the block's waits has run out.
-__device__ __forceinline__ bool marks_wait(MarksSmem& sm, uint64_t* bar, int parity) {
-    const bool ok = __all_sync(~0u, umma::mbar_wait_abort(bar, parity, kMWaitLimit, &sm.abort));
+// Wait of a whole warp for a phase of one of the block's barriers, at most `polls`
+// times; false when it or another of the block's waits has run out.
+__device__ __forceinline__ bool marks_wait(MarksSmem& sm, uint64_t* bar, int parity,
+                                           unsigned polls) {
+    const bool ok = __all_sync(~0u, umma::mbar_wait_abort(bar, parity, polls, &sm.abort));
     if (!ok) *const_cast<volatile int*>(&sm.abort) = 1;
     return ok;
 }

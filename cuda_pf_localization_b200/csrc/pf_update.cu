@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(kMThreads, 1)
                    const CObservation* __restrict__ obs, int nobs, const float* __restrict__ lm,
                    int lm_count, float sigma_r, float sigma_b, float gate,
                    float* __restrict__ ll, float2* part, unsigned* done, CycleCtl* ctl,
-                   const CycleArgs* ca) {
+                   const CycleArgs* ca, unsigned polls) {
     extern __shared__ __align__(16) unsigned char marks_smem[];
     MarksSmem& sm = *reinterpret_cast<MarksSmem*>(marks_smem);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(kMThreads, 1)
             const float2 acc = group == 0 ? marks_unit(sm, in_tensor, g, gate_max, pk)
                                           : marks_unit(sm, in_shared, g, gate_max, pk);
             const int b = k & 1, phase = (k >> 1) & 1;
-            if (k > 1 && !marks_wait(sm, &sm.summed[group][b], phase ^ 1)) {
+            if (k > 1 && !marks_wait(sm, &sm.summed[group][b], phase ^ 1, polls)) {
                 ok = false;
                 break;
             }
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kMThreads, 1)
             else if (i < n)
                 ll[i] = acc.x;
             marks_arrive(&sm.scored[group][b]);
-            ok = marks_wait(sm, &sm.ready[group], k & 1);
+            ok = marks_wait(sm, &sm.ready[group], k & 1, polls);
             if (!ok) break;
             tile = *const_cast<volatile int*>(&sm.tile[group]);
         }
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(kMThreads, 1)
         int tile = blockIdx.x + group * gridDim.x;
         for (int k = 0; tile >= 0 && tile < ntiles; ++k) {
             // the group works on tile k; prepare tile k + 1
-            if (k > 0 && !(ok = marks_wait(sm, &sm.taken[group], (k - 1) & 1))) break;
+            if (k > 0 && !(ok = marks_wait(sm, &sm.taken[group], (k - 1) & 1, polls))) break;
             if (w == 0) {
                 if (lane == 0) {
                     const int next = atomicAdd(&sm.next, 1) * (int)gridDim.x + blockIdx.x;
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(kMThreads, 1)
                 }
                 marks_arrive(&sm.claimed[group]);
             }
-            if (!(ok = marks_wait(sm, &sm.claimed[group], k & 1))) break;
+            if (!(ok = marks_wait(sm, &sm.claimed[group], k & 1, polls))) break;
             const int next = *const_cast<volatile int*>(&sm.tile[group]);
             for (int l = 32 * w + lane; next >= 0 && l < kMTile; l += 32 * kMScouts) {
                 const int i = next * kMTile + l;
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kMThreads, 1)
             marks_arrive(&sm.ready[group]);
             if (w == 0) {
                 const int b = k & 1;
-                if (!(ok = marks_wait(sm, &sm.scored[group][b], (k >> 1) & 1))) break;
+                if (!(ok = marks_wait(sm, &sm.scored[group][b], (k >> 1) & 1, polls))) break;
                 const float2 pb =
                     tile_softmax_partial(sm.ll[group][b], min(kMTile, n - tile * kMTile));
                 if (lane == 0) part[tile] = pb;
@@ -402,7 +402,10 @@ __global__ void __launch_bounds__(kMThreads, 1)
     __threadfence();
     const float2 ms = softmax_combine(part, ntiles);
     if (tid == 0) {
-        softmax_commit(ms, ctl);
+        // after a wait has run out some tiles have the log-likelihoods and partials of
+        // another call, whose weights could be anything: the cloud stays uniform
+        const bool whole = (__ldcg(&ctl->err) & ERR_SPIN_TIMEOUT) == 0;
+        softmax_commit(whole ? ms : make_float2(0.0f, 0.0f), ctl);
         *done = 0u;
     }
 }
@@ -419,7 +422,7 @@ int launch_marks(PfHandle* h, const PredictArgs& pa, const CObservation* d_obs, 
     PFB_CK(launch_pdl(k_weight_marks<kPredict>, grid, kMThreads, sizeof(MarksSmem), h->stream,
                       plane_set(h), h->n, h->seed, pa, d_obs, nobs, h->d_lm, h->lm_count, sigma_r,
                       sigma_b, gate, h->d_ll, reinterpret_cast<float2*>(h->d_part), h->d_done + 0,
-                      h->d_ctl, dargs));
+                      h->d_ctl, dargs, h->wait_polls));
     return 0;
 }
 

@@ -205,6 +205,13 @@ int pfc_cycle_result(void* h, double* est_out);
  * Both give identical results.  Cycles run with per-kernel profiling
  * (pfc_profile) always use direct launches. */
 int pfc_set_graph(void* h, int on);
+/* Test hook for the bounded waits of the weighting that rotates every landmark
+ * once: polls before a wait gives up (0: every wait runs out at once; -1
+ * restores the default of 2^24).  A wait that runs out leaves the weights
+ * uniform and sets an error bit: the call that waits for the result returns -1
+ * with "a device wait timed out" in pfc_last_error_message(), and so do the
+ * handle's later ones until pfc_init. */
+int pfc_set_wait_test(void* h, int polls);
 /* Cycle graphs captured by this handle so far (a test hook: a graph whose
  * buffers have been replaced has to be captured again); -1 without a handle. */
 long long pfc_graph_captures(void* h);
