@@ -218,8 +218,9 @@ int wait_estimate(PfHandle* h) {
     h->est_inflight = false;
     h->est_valid = true;
     if (h->last_obs_dev) {
-        h->dev_obs_mixed = h->dev_obs_mixed || !h->h_ctl->obs_cart;
-        h->dev_obs_cart = !h->dev_obs_mixed;
+        h->dev_cart_run = h->h_ctl->obs_cart ? std::min(h->dev_cart_run + 1, 1)
+                                             : -PfHandle::kMixedRun;
+        h->last_obs_dev = false;  // counted
     }
     return device_error(h);
 }
@@ -541,6 +542,8 @@ int init_particles(PfHandle* h, int n, unsigned int seed, int n_pad) {
     h->gen = 0;
     h->pending_predict = false;
     h->est_valid = h->est_inflight = false;
+    h->dev_cart_run = 0;
+    h->last_obs_dev = false;
     h->anc_valid = false;
     h->prefix_valid = false;
     const size_t np = (size_t)h->n_pad;
@@ -805,7 +808,8 @@ int pfc_cycle_device(void* hv, const PfcOdom* odom, const void* d_obs, int nobs,
     if (nobs > h->cap_obs) nobs = h->cap_obs;
     if (!d_obs) nobs = 0;
     h->last_obs_dev = nobs > 0;
-    if (run_cycle(h, odom, static_cast<const CObservation*>(d_obs), nobs, h->dev_obs_cart, prm))
+    if (run_cycle(h, odom, static_cast<const CObservation*>(d_obs), nobs, h->dev_cart_run > 0,
+                  prm))
         return -1;
     if (!est_out) return 0;
     return finish_cycle(h, est_out);

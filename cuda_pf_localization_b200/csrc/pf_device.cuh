@@ -277,6 +277,18 @@ __device__ __forceinline__ float comp(const float4& v, int c) {
     return c == 0 ? v.x : (c == 1 ? v.y : (c == 2 ? v.z : v.w));
 }
 
+// Observation o into slot `slot` of the staged arrays.
+__device__ __forceinline__ void stage_one(const CObservation& o, const float* __restrict__ lm,
+                                          int slot, float4* s_a, float4* s_b, float4* s_p) {
+    const float lx = lm[3 * o.id], ly = lm[3 * o.id + 1], lz = lm[3 * o.id + 2];
+    s_a[slot] = make_float4(lx, ly, lz, __int_as_float(o.mode == 0 ? 1 : 2));
+    s_b[slot] = make_float4(o.dx, o.dy, o.dz, o.range);
+    // broadcast pairs for the packed two-particle path
+    s_p[3 * slot] = make_float4(lx, lx, ly, ly);
+    s_p[3 * slot + 1] = make_float4(lz, lz, -o.dx, -o.dx);
+    s_p[3 * slot + 2] = make_float4(-o.dy, -o.dy, -o.dz, -o.dz);
+}
+
 // Stage observations [c0, c0 + cn) into shared memory, dropping the ones
 // whose id is outside the landmark table (the reference skips them with
 // `continue`, pf_kernels.cu:242) and keeping the order of the rest, so the
@@ -306,13 +318,7 @@ __device__ __forceinline__ int stage_chunk(const CObservation* __restrict__ obs,
     }
     if (keep) {
         const int slot = off + __popc(ballot & ((1u << lane) - 1u));
-        const float lx = lm[3 * o.id], ly = lm[3 * o.id + 1], lz = lm[3 * o.id + 2];
-        s_a[slot] = make_float4(lx, ly, lz, __int_as_float(o.mode == 0 ? 1 : 2));
-        s_b[slot] = make_float4(o.dx, o.dy, o.dz, o.range);
-        // broadcast pairs for the packed two-particle path
-        s_p[3 * slot] = make_float4(lx, lx, ly, ly);
-        s_p[3 * slot + 1] = make_float4(lz, lz, -o.dx, -o.dx);
-        s_p[3 * slot + 2] = make_float4(-o.dy, -o.dy, -o.dz, -o.dz);
+        stage_one(o, lm, slot, s_a, s_b, s_p);
     }
     *all_cart = cart != 0;
     __syncthreads();
@@ -571,10 +577,36 @@ __device__ __forceinline__ float2 softmax_combine(const float2* part, int G) {
     return make_float2(M, s_r);
 }
 
+// The staged observations [0, cn) of any kind against two particles, added to acc in
+// their order.
+__device__ __forceinline__ void packed_terms(const PackedPose& pk, const GateConsts& g,
+                                             const float4* s_a, const float4* s_b,
+                                             const float4* s_p, int cn, float2& acc) {
+    PackedBearing gb;
+    gb.ninv_r = both(-g.inv2rr);
+    gb.ninv_b = both(-g.inv2bb);
+    gb.rng_gate2 = g.gate > 0.0f ? g.rng_gate2 : INFINITY;
+    gb.brg_gate2 = g.gate > 0.0f ? g.brg_gate2 : INFINITY;
+    gb.out = g.half_out;
+    const float cart_gate2 = g.gate > 0.0f ? g.cart_gate2 : INFINITY;
+#pragma unroll 2
+    for (int k = 0; k < cn; ++k) {
+        const float4 A = s_p[3 * k], B = s_p[3 * k + 1], C = s_p[3 * k + 2];
+        if (__float_as_int(s_a[k].w) == 1) {
+            const float2 r2 = packed_r2(pk, A, B, C);
+            const float2 t = __fmul2_rn(r2, gb.ninv_r);
+            acc = __fadd2_rn(acc, make_float2(r2.x > cart_gate2 ? g.cart_out : t.x,
+                                              r2.y > cart_gate2 ? g.cart_out : t.y));
+        } else {
+            packed_bearing(pk, gb, A, B, C, s_b[k].w, acc);
+        }
+    }
+}
+
 // Gated log-likelihoods of two particles (p0,q0) and (p1,q1) against nobs
 // observations, staged kObsChunk at a time into shared memory (the whole
-// block takes part).  use_packed selects the packed f32x2 paths; every path produces the reference's roundings.  Returns
-// whether every observation kept was Cartesian.
+// block takes part).  use_packed selects the packed f32x2 paths; every path produces
+// the reference's roundings.  Returns whether every observation kept was Cartesian.
 __device__ __forceinline__ bool weight_two(
     const CObservation* __restrict__ obs, int nobs, const float* __restrict__ lm,
     int lm_count, float sigma_r, float sigma_b, float gate, float3 p0, Quat q0,
@@ -596,25 +628,7 @@ __device__ __forceinline__ bool weight_two(
         cart = cart && all_cart;
         if (!all_cart && use_packed) {
             float2 acc = make_float2(acc0, acc1);
-            PackedBearing gb;
-            gb.ninv_r = ninv;
-            gb.ninv_b = both(-g.inv2bb);
-            gb.rng_gate2 = gate > 0.0f ? g.rng_gate2 : INFINITY;
-            gb.brg_gate2 = gate > 0.0f ? g.brg_gate2 : INFINITY;
-            gb.out = g.half_out;
-            const float cart_gate2 = gate > 0.0f ? g.cart_gate2 : INFINITY;
-#pragma unroll 2
-            for (int k = 0; k < cn; ++k) {
-                const float4 A = s_p[3 * k], B = s_p[3 * k + 1], C = s_p[3 * k + 2];
-                if (__float_as_int(s_a[k].w) == 1) {
-                    const float2 r2 = packed_r2(pk, A, B, C);
-                    const float2 t = __fmul2_rn(r2, ninv);
-                    acc = __fadd2_rn(acc, make_float2(r2.x > cart_gate2 ? g.cart_out : t.x,
-                                                      r2.y > cart_gate2 ? g.cart_out : t.y));
-                } else {
-                    packed_bearing(pk, gb, A, B, C, s_b[k].w, acc);
-                }
-            }
+            packed_terms(pk, g, s_a, s_b, s_p, cn, acc);
             acc0 = acc.x;
             acc1 = acc.y;
         } else if (all_cart && use_packed) {

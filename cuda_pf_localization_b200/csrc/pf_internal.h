@@ -241,10 +241,13 @@ struct PfHandle {
     double* d_part = nullptr;           // per-block partials (max over uses)
     int part_cap = 0;                   // doubles in d_part
     unsigned long long* d_part_u64 = nullptr;  // per-block integer partials
-    // observations in device memory, which the host has not seen: Cartesian in the
-    // last cycle that was waited for (0 until then), never again after a cycle
-    // that was not
-    bool dev_obs_cart = false, dev_obs_mixed = false, last_obs_dev = false;
+    // Observations in device memory, which the host has not seen, are taken to be
+    // Cartesian while this is positive: the cycles of the cloud that were waited for
+    // and were, in a row (up to 1), less kMixedRun after one that was not.  A wrong
+    // guess costs a sixth to a third of a weighting, a guess not made a third.
+    static constexpr int kMixedRun = 8;
+    int dev_cart_run = 0;
+    bool last_obs_dev = false;
     bool prefix_valid = false;  // ctl w_total_fx and d_wprefix describe the
                                 // current weights
     unsigned* d_done = nullptr;         // last-block counters

@@ -51,7 +51,7 @@ static_assert(kMMarks * kMColumns == 512, "all columns of tensor memory");
 struct MarksSmem {
     // [marker][slot][x, y, z][lane]: landmarks in the frames of the lane's particles
     float2 pred[kMMarkers][kMMarks][3][32];
-    float4 rec[2 * kMObs];  // (-ox, -oy, -oz, slot in columns); weight_tiles takes two each
+    float4 rec[kMObs];  // (-ox, -oy, -oz, slot in columns)
     float4 mark_xy[kMMarks];  // (lx, lx, ly, ly)
     float2 mark_z[kMMarks];
     float pose[kMGroups][7][kMTile];

@@ -203,7 +203,12 @@ __device__ __forceinline__ float2 tile_softmax_partial(const float* s_ll, int co
     return make_float2(bm, sb);
 }
 
-// Any observations, a particle per thread: k_weight_marks' way with bearings.
+// Any observations: k_weight_marks' way with bearings, k_weight's arithmetic by four
+// groups of kWThreads threads, a 256-particle tile each at a time.  Sixteen warps an SM
+// where k_weight has twenty, and a block's tiles do not divide evenly: 1M x 64 / 256, one
+// bearing among them, 395 us against 315, every third one 556 and 478, all of them 880
+// and 752 (a particle a thread with scalar arithmetic on half of the block: 2.3 to 2.9
+// times k_weight's).
 template <bool kPredict>
 __device__ __noinline__ void weight_tiles(MarksSmem& sm, const Planes& s, int n, uint64_t seed,
                                           const PredictArgs& pa,
@@ -211,45 +216,61 @@ __device__ __noinline__ void weight_tiles(MarksSmem& sm, const Planes& s, int n,
                                           const float* __restrict__ lm, int lm_count,
                                           float sigma_r, float sigma_b, float gate,
                                           float* __restrict__ ll, float2* part) {
-    constexpr int kTile = kMTile;
+    constexpr int kGroups = kMThreads / kWThreads;
+    static_assert(sizeof sm.pred >= 5 * kMObs * sizeof(float4), "the staged observations");
+    static_assert(sizeof sm.ll >= kGroups * kMTile * sizeof(float), "a tile a group");
+    float4* const s_a = reinterpret_cast<float4*>(sm.pred);
+    float4 *const s_b = s_a + kMObs, *const s_p = s_b + kMObs;
     const GateConsts g = gate_consts(sigma_r, sigma_b, gate);
-    const int tid = threadIdx.x;
-    __syncthreads();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int group = tid / kWThreads, t = tid % kWThreads;
+    float* const s_ll = &sm.ll[0][0][0] + group * kMTile;
+    auto group_sync = [&]() {
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(kWThreads) : "memory");
+    };
+    CObservation o{};
+    bool keep = false;
     if (tid < nobs) {
-        const CObservation o = obs[tid];
-        const bool keep = o.id >= 0 && o.id < lm_count;
-        const float* l = lm + 3 * (keep ? o.id : 0);
-        sm.rec[2 * tid] = make_float4(l[0], l[1], l[2],
-                                      __int_as_float(!keep ? 0 : o.mode == 0 ? 1 : 2));
-        sm.rec[2 * tid + 1] = make_float4(o.dx, o.dy, o.dz, o.range);
+        o = obs[tid];
+        keep = o.id >= 0 && o.id < lm_count;
     }
+    const unsigned kept = __ballot_sync(~0u, keep);
+    int at = __popc(kept & ((1u << lane) - 1u));
+    for (int k = 0; k < warp; ++k) at += sm.warp_count[k];  // left by marks_build
+    if (keep) stage_one(o, lm, at, s_a, s_b, s_p);
+    const int cn = sm.kept;
     __syncthreads();
-    for (int tile = blockIdx.x; tile * kTile < n; tile += gridDim.x) {
-        const int i = tile * kTile + tid;
-        if (tid < kTile && i < n) {
-            float3 p;
-            Quat q;
-            load_pose(s, i, p, q);
-            if (kPredict) {
-                apply_predict(pa, seed, i, p, q);
-                store_pose(s, i, p, q);
+    for (int tile = blockIdx.x + group * gridDim.x; (long long)tile * kMTile < n;
+         tile += kGroups * gridDim.x) {
+        const int i0 = tile * kMTile + t;
+        float3 p[2];
+        Quat q[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = i0 + h * kWThreads;
+            p[h] = make_float3(0.f, 0.f, 0.f);
+            q[h] = {1.f, 0.f, 0.f, 0.f};
+            if (i < n) {
+                load_pose(s, i, p[h], q[h]);
+                if (kPredict) {
+                    apply_predict(pa, seed, i, p[h], q[h]);
+                    store_pose(s, i, p[h], q[h]);
+                }
             }
-            const Quat qc = q_conjugate(q);
-            float acc = 0.0f;
-            for (int k = 0; k < nobs; ++k) {
-                const float4 a = sm.rec[2 * k];
-                const int kind = __float_as_int(a.w);
-                if (kind != 0) obs_loglik(g, p, qc, a, sm.rec[2 * k + 1], kind, acc);
-            }
-            ll[i] = acc;
-            sm.ll[0][0][tid] = acc;
         }
-        __syncthreads();
-        if (tid < 32) {
-            const float2 pb = tile_softmax_partial(sm.ll[0][0], min(kTile, n - tile * kTile));
-            if (tid == 0) part[tile] = pb;
+        const PackedPose pk = pack_pose(p[0], q_conjugate(q[0]), p[1], q_conjugate(q[1]));
+        float2 acc = make_float2(0.f, 0.f);
+        packed_terms(pk, g, s_a, s_b, s_p, cn, acc);
+        if (i0 < n) ll[i0] = acc.x;
+        if (i0 + kWThreads < n) ll[i0 + kWThreads] = acc.y;
+        s_ll[t] = acc.x;
+        s_ll[t + kWThreads] = acc.y;
+        group_sync();
+        if (t < 32) {
+            const float2 pb = tile_softmax_partial(s_ll, min(kMTile, n - tile * kMTile));
+            if (t == 0) part[tile] = pb;
         }
-        __syncthreads();
+        group_sync();
     }
 }
 

@@ -155,3 +155,69 @@ def test_arguments_checked(kernels):
         assert kernels.pfc_set_wait_test(pf.h, -2) == -1
     finally:
         pf.close()
+
+
+# Observations in device memory: a cycle takes the kernel when the host's guess is that
+# they are Cartesian, which the last call of each history shows.
+@pytest.mark.parametrize("history,guess", [
+    ("", False), ("c", True), ("m", False), ("cm", False), ("cm" + 8 * "c", False),
+    ("cm" + 9 * "c", True), (20 * "c" + "m" + 8 * "c", False), ("m" + 9 * "c", True),
+    ("m" + 8 * "c" + "m" + 9 * "c", True), ("mmm" + 9 * "c", True), ("ch", True), ("h", False),
+    ("mh" + 9 * "c", True), ("cI", False), ("mIc", True), ("cmI", False)])
+def test_guess_follows_the_cycles(kernels, history, guess):
+    n = 100_001
+    lm, rows = _rows(24, 256)
+    one = _rows(24, 256, "one")[1]
+    pf = _filter(kernels, n, lm)
+    try:
+        for step in history:
+            if step == "I":
+                assert kernels.pfc_init(pf.h, n, 5) == 0
+                _prior(pf)
+            else:  # Cartesian or mixed from the device, Cartesian from the host
+                assert _cycle(pf, one if step == "m" else rows, step != "h")[0] == 0
+        assert kernels.pfc_set_wait_test(pf.h, 0) == 0
+        assert _cycle(pf, rows, True)[0] == (-1 if guess else 0)
+    finally:
+        pf.close()
+
+
+@pytest.mark.parametrize("mode", ["one", "bearing"])
+@pytest.mark.parametrize("landmarks,nobs,n,gate", [
+    (64, 256, 83_334, 3.0), (1, 96, 168_447, 0.0), (24, 131, 151_553, 2.5), (5, 256, 606_209, 3.0)])
+def test_a_wrong_guess_gives_the_same_bits(kernels, mode, landmarks, nobs, n, gate):
+    """A Cartesian cycle, then one that is not, in the kernel that guesses (151 552 and
+    606 208 particles fill 148 blocks' four tiles once and four times) and in the scalar
+    one; unknown ids among the observations, and poses that are not finite."""
+    import torch
+    lm, cart = _rows(landmarks, nobs)
+    other = _rows(landmarks, nobs, mode, seed=4)[1]
+    other[::7, 0] = landmarks + 2
+    other[3::11, 0] = -1
+    rng = np.random.default_rng(2)
+    pos = rng.normal(0, 0.3, (n, 3)).astype(np.float32)
+    quat = rng.normal(0, 0.1, (n, 4)).astype(np.float32) + np.float32([1, 0, 0, 0])
+    pos[7], quat[n - 1] = np.nan, np.inf
+    got = []
+    for variant in (0, 1):
+        pf = _filter(kernels, n, lm)
+        try:
+            assert kernels.pfc_set_weight_kernel(pf.h, variant) == 0
+            assert _cycle(pf, cart, True)[0] == 0
+            assert kernels.pfc_set_state(pf.h, pkg.fptr(pos), pkg.fptr(quat), None) == 0
+            odom = pkg.PfcOdom()
+            odom.t[:], odom.q[:] = [0.0] * 3, [1.0, 0.0, 0.0, 0.0]
+            odom.tstd[:], odom.rstd[:] = [0.02] * 3, [0.01] * 3
+            prm = pkg.PfcCycleParams(0.5, 0.2, gate, 0.5, 0.01, 0)
+            d_obs = torch.from_numpy(pkg.cobs_records(other).view(np.uint8).copy()).cuda()
+            torch.cuda.synchronize()
+            est, ll = np.zeros(pkg.PFC_EST_LEN), np.zeros(n, np.float32)
+            assert kernels.pfc_cycle_device(pf.h, C.byref(odom), C.c_void_p(d_obs.data_ptr()),
+                                            nobs, C.byref(prm), pkg.dptr(est)) == 0
+            assert kernels.pfc_get_ll(pf.h, pkg.fptr(ll)) == 0
+            got.append((est, ll, *pf.snapshot()))
+        finally:
+            pf.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b, equal_nan=True)
+    assert len(np.unique(got[0][1])) > n // 100
