@@ -890,9 +890,13 @@ int ensure_scan(GlHandle* h, const float* scan, int nrays) {
 // beside them.  The stepping is bound by issued instructions, so the shape with
 // the most warps on an SM is taken: two blocks of up to 24, else one of up to
 // 32 (20 011 hypotheses x 271 rays on 401 x 299 cells, which one block an SM
-// holds: 629 us at 24 warps before ray_chunk, 316 at 32 with it).  Where the padded grid leaves room for fewer than kMinSmemWarps it stays in
-// global memory and its cells come through L1; so it does where a ray could take
-// more than 8192 steps, which the shared-memory stepping does not count.
+// holds: 629 us at 24 warps before ray_chunk, 316 at 32 with it).  Where the padded
+// grid leaves room for fewer than kMinSmemWarps it stays in global memory; so it does
+// where a ray could take more than 8192 steps, which the shared-memory stepping does
+// not count.  Its cells then come through L1, which has what the slots leave of the
+// SM's memory: two blocks of 24 warps where their slots fit, else one of 24 and not
+// two of fewer (20 000 hypotheses on 600 x 600 cells, 600 rays: 4.7 ms and 9.0 with
+// two blocks, 1000 rays 8.0 and 12.0).
 constexpr int kSmBytes = 233472 - 2 * 1088;  // of an SM, less what each block reserves
 constexpr int kMaxSlotBytes = 200 * 1024;    // ray slots of 24 warps and the scan
 constexpr int kMinSmemWarps = 10;
@@ -922,10 +926,9 @@ bool score_plan(const GlHandle* h, int nrays, int nscan, ScorePlan* p) {
         p->warps = p->per_sm == 2 ? pair : solo;
         p->bytes = (size_t)(grid + scan + slot * p->warps);
     } else {
-        const int w2 = fit(scan, 2, kPairThreads / 32), w1 = fit(scan, 1, kPairThreads / 32);
-        p->per_sm = w2 > 0 ? 2 : 1;
-        p->warps = w2 > 0 ? w2 : w1;
+        p->warps = kPairThreads / 32;
         p->bytes = (size_t)(scan + slot * p->warps);
+        p->per_sm = 2 * (long long)p->bytes <= kSmBytes ? 2 : 1;
     }
     return true;
 }
