@@ -109,10 +109,9 @@ __device__ __forceinline__ Offsets offsets(const CycleCtl* ctl, int n, int use_u
     return o;
 }
 
-// Injection draws of one tile, in shared memory: local output, draw index,
-// jitter, the next listed draw on the same output.
+// Injection draws of one tile, in shared memory: draw index, jitter, the next
+// listed draw on the same output.
 struct InjList {
-    int loc[kThreads];
     int j[kThreads];
     float jx[kThreads], jy[kThreads], jz[kThreads];
     int next[kThreads];
@@ -140,29 +139,6 @@ __device__ __forceinline__ void apply_chain(const InjList& L, int head, float& x
             if (L.j[e] > last && (best < 0 || L.j[e] < L.j[best])) best = e;
         if (best < 0) break;
         apply_draw(L, best, x, y, z, d);
-        last = L.j[best];
-    }
-}
-
-// Apply to the group of outputs [l0, l0 + kGroup), in ascending draw order,
-// the listed draws (m entries, any order) that hit it; the exact change of
-// every position value goes to d[0..2].
-__device__ __forceinline__ void apply_draws(const InjList& L, int m, int l0,
-                                            float (&x)[kGroup], float (&y)[kGroup],
-                                            float (&z)[kGroup], double (&d)[kCorrN]) {
-    int hits = 0;
-    for (int e = 0; e < m; ++e) hits += (unsigned)(L.loc[e] - l0) < (unsigned)kGroup;
-    int last = -1;
-    for (int h = 0; h < hits; ++h) {
-        int best = -1;
-        for (int e = 0; e < m; ++e)
-            if ((unsigned)(L.loc[e] - l0) < (unsigned)kGroup && L.j[e] > last &&
-                (best < 0 || L.j[e] < L.j[best]))
-                best = e;
-        const int r = L.loc[best] - l0;
-#pragma unroll
-        for (int q = 0; q < kGroup; ++q)
-            if (q == r) apply_draw(L, best, x[q], y[q], z[q], d);
         last = L.j[best];
     }
 }
@@ -359,7 +335,6 @@ __global__ void __launch_bounds__(kThreads, 4)
     if (ca) gen = ca->gen;
     __shared__ __align__(16) GatherSmem sm;
     __shared__ int s_wmax[kThreads / 32];
-    __shared__ int s_m;
     __shared__ double s_out[kEstN];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // the tiles go to blocks 1.. (block 0 combines the sums), or to block 0 when it is
@@ -426,19 +401,18 @@ __global__ void __launch_bounds__(kThreads, 4)
         // by scanning every draw in rounds below
         const bool overflow = cnt > inj_cap;
         const int m = overflow ? 0 : cnt;
-        if (m > 0) {
+        auto list = [&](int j, const InjDraw& d) {
+            s_inj.j[tid] = j;
+            s_inj.jx[tid] = d.jx;
+            s_inj.jy[tid] = d.jy;
+            s_inj.jz[tid] = d.jz;
+            s_inj.next[tid] = atomicExch(&sm.head[d.idx - (int)o0], tid);
+        };
+        if (cnt > 0) {
             int4* h4 = reinterpret_cast<int4*>(sm.head);
             h4[tid] = h4[tid + kThreads] = make_int4(-1, -1, -1, -1);
             __syncthreads();
-            if (tid < m) {
-                const InjDraw d = inj_draw(lcg1, gen, bj, n);
-                const int loc = d.idx - (int)o0;
-                s_inj.j[tid] = bj;
-                s_inj.jx[tid] = d.jx;
-                s_inj.jy[tid] = d.jy;
-                s_inj.jz[tid] = d.jz;
-                s_inj.next[tid] = atomicExch(&sm.head[loc], tid);
-            }
+            if (tid < m) list(bj, inj_draw(lcg1, gen, bj, n));
         }
         // ancestors of outputs [8t, 8t + 8): running maximum of the markers
         // (thread, then block); the markers read are reset for the next one
@@ -483,52 +457,34 @@ __global__ void __launch_bounds__(kThreads, 4)
             }
             // the tile's injection draws on these outputs (the bucket's, or
             // all draws in rounds on a bucket overflow)
-            if (m > 0) {
+            auto apply_listed = [&]() {
                 const int4 hd = *reinterpret_cast<const int4*>(&sm.head[l0]);
                 if (hd.x >= 0) apply_chain(s_inj, hd.x, v[0][0], v[1][0], v[2][0], corr);
                 if (hd.y >= 0) apply_chain(s_inj, hd.y, v[0][1], v[1][1], v[2][1], corr);
                 if (hd.z >= 0) apply_chain(s_inj, hd.z, v[0][2], v[1][2], v[2][2], corr);
                 if (hd.w >= 0) apply_chain(s_inj, hd.w, v[0][3], v[1][3], v[2][3], corr);
-            }
-            if (overflow) {
-                // rounds of kInjChunk draws, the round's hits on this tile
-                // compacted in draw order and applied in that order
-                // (block-uniform: every thread takes the same rounds)
-                for (int base = 0; base < k_inj; base += kInjChunk) {
-                    __syncthreads();
-                    const int j = base + tid;
-                    InjDraw d{};
-                    bool hit = false;
+            };
+            // rounds of kInjChunk draws in ascending order, those on this tile listed
+            // like a bucket's (block-uniform: every thread takes the same rounds)
+            const int rounds = overflow ? ceil_div(k_inj, kInjChunk) : m > 0 ? 1 : 0;
+            for (int q = 0; q < rounds; ++q) {
+                InjDraw d{};
+                bool hit = false;
+                if (overflow) {
+                    const int j = q * kInjChunk + tid;
                     if (j < k_inj) {
                         d = inj_draw(lcg1, gen, j, n);
                         hit = d.idx >= o0 && d.idx < o0 + kTile;
+                        if (hit) list(j, d);
                     }
-                    const unsigned bal = __ballot_sync(~0u, hit);
-                    if (lane == 0) s_inj.j[warp] = __popc(bal);  // counts, then offsets
-                    __syncthreads();
-                    if (tid == 0) {
-                        int off = 0;
-                        for (int k = 0; k < kThreads / 32; ++k) {
-                            const int cw = s_inj.j[k];
-                            s_inj.j[k] = off;
-                            off += cw;
-                        }
-                        s_m = off;
-                    }
-                    __syncthreads();
-                    const int off = s_inj.j[warp] + __popc(bal & ((1u << lane) - 1u));
-                    __syncthreads();
-                    if (hit) {
-                        s_inj.loc[off] = d.idx - (int)o0;
-                        s_inj.j[off] = j;
-                        s_inj.jx[off] = d.jx;
-                        s_inj.jy[off] = d.jy;
-                        s_inj.jz[off] = d.jz;
-                    }
-                    __syncthreads();
-                    apply_draws(s_inj, s_m, l0, v[0], v[1], v[2], corr);
+                    if (!__syncthreads_or(hit)) continue;
                 }
-                __syncthreads();
+                apply_listed();
+                if (overflow) {
+                    __syncthreads();
+                    if (hit) sm.head[d.idx - (int)o0] = -1;
+                    __syncthreads();
+                }
             }
             if (ib + kGroup <= n) {
 #pragma unroll
