@@ -281,7 +281,7 @@ void cycle_graph_key(const PfHandle* h, const PfcCycleParams* prm, int kinj,
     k[6] = f2l(prm->gate);
     k[7] = e;
     k[8] = f2l(prm->random_inject_ratio);
-    k[9] = h->weight_variant;
+    k[9] = 2 * h->weight_variant + (h->lm_wild ? 1 : 0);
     k[10] = h->record_anc ? 1 : 0;
     k[11] = kinj > 0 ? (long long)(uintptr_t)h->d_inj_bucket : 0;
     k[12] = kinj > 0 ? h->inj_cap : 0;
@@ -590,8 +590,10 @@ int pfc_upload_landmarks(void* hv, const float* xyz, int count) {
     // valid-id bound only grows otherwise.
     if (count == 0) {
         h->lm_count = 0;
+        h->lm_wild = false;
         return 0;
     }
+    h->lm_wild = !tame_landmarks(xyz, count) || (h->lm_wild && count < h->lm_count);
     if (count > h->lm_cap) {
         PFB_CK(cudaStreamSynchronize(h->stream));
         cudaFree(h->d_lm);

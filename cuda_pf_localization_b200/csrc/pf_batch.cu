@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kWThreads, 6)
     k_b_weight(Arena A, const BFilter* __restrict__ F, const BTile* __restrict__ T,
                BCtl* C, const PfcBatchCycle* __restrict__ cyc,
                const CObservation* __restrict__ obs, const float* __restrict__ lm,
-               float2* __restrict__ wpart, int use_packed) {
+               float2* __restrict__ wpart, int arith) {
     const BTile t = T[blockIdx.x];
     const BFilter& fl = F[t.f];
     BCtl* c = C + t.f;
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(kWThreads, 6)
     }
     float acc0, acc1;
     weight_two(obs + in.obs_off, nobs, lm + 3 * (size_t)fl.lm_off, fl.lm_count,
-               fl.sigma_r, fl.sigma_b, fl.gate, p0, q0, p1, q1, use_packed, acc0,
+               fl.sigma_r, fl.sigma_b, fl.gate, p0, q0, p1, q1, arith, acc0,
                acc1);
     float* ll = A.ll + fl.off;
     if (v0) ll[i0] = acc0;
@@ -978,6 +978,7 @@ struct BatchHandle {
     std::vector<BFilter> filters;
     std::vector<int> est_tile;  // per bucket
     int use_packed = 1;
+    bool lm_wild = false;  // a landmark is not tame (tame_landmark)
     long long arena = 0;         // particles incl. padding
     float* d_planes = nullptr;   // 2 x 7 planes + ll + w
     Arena A{};
@@ -1104,7 +1105,10 @@ int launch_est_covs(BatchHandle* h) {
 int enqueue_cycle(BatchHandle* h) {
     cudaStream_t s = h->stream;
     PFB_CK(launch_pdl(k_b_weight, h->n_wt, kWThreads, 0, s, h->A, h->d_F, h->d_wt, h->d_C,
-                      h->d_cyc, h->d_obs, h->d_lm, h->d_wpart, h->use_packed));
+                      h->d_cyc, h->d_obs, h->d_lm, h->d_wpart,
+                      !h->use_packed ? ARITH_SCALAR
+                      : h->lm_wild   ? ARITH_PACKED_WILD
+                                     : ARITH_PACKED));
     PFB_CK(launch_pdl(k_b_ess, h->n_et, kThreads, 0, s, h->A, h->d_F, h->d_et, h->d_C,
                       h->d_epart, h->d_eupart));
     PFB_CK(launch_pdl(k_b_resample, h->n_rt, kThreads, 0, s, h->A, h->d_F, h->d_rt, h->d_C,
@@ -1403,6 +1407,7 @@ int pfc_batch_upload_landmarks(void* p, const float* xyz, const int* counts) {
         tot += counts[f];
     }
     if (tot > 0 && !xyz) return -1;
+    h->lm_wild = !tame_landmarks(xyz, tot);
     if (tot > h->lm_total) {
         cudaFree(h->d_lm);
         h->d_lm = nullptr;

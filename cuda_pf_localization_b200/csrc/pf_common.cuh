@@ -267,6 +267,20 @@ __host__ __device__ __forceinline__ uint64_t composite_key(float caer,
     return ((uint64_t)u << 32) | (uint64_t)idx;
 }
 
+// ---------------------------------------------------------------- tame values
+// Landmarks and positions below kTameCoord, and quaternion components below kTameQuat,
+// leave a factor of two in the rotation's products short of overflow.
+constexpr float kTameCoord = 0x1p100f, kTameQuat = 0x1p20f;
+__host__ __device__ __forceinline__ bool tame_landmark(float x, float y, float z) {
+    return fabsf(x) < kTameCoord && fabsf(y) < kTameCoord && fabsf(z) < kTameCoord;
+}
+inline bool tame_landmarks(const float* xyz, long long count) {
+    bool tame = true;
+    for (long long k = 0; k < count; ++k)
+        tame = tame && tame_landmark(xyz[3 * k], xyz[3 * k + 1], xyz[3 * k + 2]);
+    return tame;
+}
+
 // ------------------------------------------------------------------ sizes
 __host__ __device__ __forceinline__ int ceil_div(int a, int b) {
     return (a + b - 1) / b;

@@ -325,24 +325,6 @@ __device__ __forceinline__ int stage_chunk(const CObservation* __restrict__ obs,
     return total;
 }
 
-// Gated Cartesian term of the reference (pf_kernels.cu:247-252) for the
-// specialised all-Cartesian loop; gate > 0 is hoisted out as kGated.
-template <bool kGated>
-__device__ __forceinline__ void cart_term(const GateConsts& g, float3 p,
-                                          const Quat& qc, float4 a, float4 b,
-                                          float& acc) {
-    float3 d = make_float3(a.x - p.x, a.y - p.y, a.z - p.z);
-    float3 pred = q_rotate(qc, d);
-    const float ex = pred.x - b.x, ey = pred.y - b.y, ez = pred.z - b.z;
-    const float r2 = sq3(ex, ey, ez);
-    // The reference rounds the product and the sum separately in both the
-    // gated and the ungated case.
-    if (kGated)
-        acc = __fadd_rn(acc, (r2 > g.cart_gate2) ? g.cart_out : __fmul_rn(-r2, g.inv2rr));
-    else
-        acc = __fadd_rn(acc, __fmul_rn(-r2, g.inv2rr));
-}
-
 // ---------------------------------------------------------- packed path
 // The Cartesian term evaluated for two particles at once with packed f32x2
 // arithmetic.  nvcc compiles the reference expression (q_rotate + squared
@@ -384,6 +366,17 @@ __device__ __forceinline__ PackedPose pack_pose(float3 p0, const Quat& c0,
     k.m6 = make_float2(2.f * k.k6.x, 2.f * k.k6.y);
     k.w2 = make_float2(2.f * c0.w, 2.f * c1.w);
     return k;
+}
+
+// The doubled coefficients give the reference's bits unless 2t' overflows where the
+// products with t' do not: for landmarks and positions below kTameCoord and quaternion
+// components below kTameQuat t' stays below 2^123.
+__device__ __forceinline__ bool tame_pose(const PackedPose& k) {
+    auto top = [](float2 a, float2 b) {
+        return max_nan(max_nan(fabsf(a.x), fabsf(a.y)), max_nan(fabsf(b.x), fabsf(b.y)));
+    };
+    return max_nan(top(k.npx, k.npy), top(k.npz, k.npz)) < kTameCoord &&
+           max_nan(top(k.k2, k.k4), top(k.k6, k.w2)) < kTameQuat;
 }
 
 // A landmark (broadcast pairs A = (lx,lx,ly,ly), z = (lz,lz)) in the body frames of
@@ -578,7 +571,8 @@ __device__ __forceinline__ float2 softmax_combine(const float2* part, int G) {
 }
 
 // The staged observations [0, cn) of any kind against two particles, added to acc in
-// their order.
+// their order.  With bearings among them for tame landmarks and poses only, else
+// scalar_terms.
 __device__ __forceinline__ void packed_terms(const PackedPose& pk, const GateConsts& g,
                                              const float4* s_a, const float4* s_b,
                                              const float4* s_p, int cn, float2& acc) {
@@ -603,83 +597,105 @@ __device__ __forceinline__ void packed_terms(const PackedPose& pk, const GateCon
     }
 }
 
-// Gated log-likelihoods of two particles (p0,q0) and (p1,q1) against nobs
-// observations, staged kObsChunk at a time into shared memory (the whole
-// block takes part).  use_packed selects the packed f32x2 paths; every path produces
-// the reference's roundings.  Returns whether every observation kept was Cartesian.
-__device__ __forceinline__ bool weight_two(
-    const CObservation* __restrict__ obs, int nobs, const float* __restrict__ lm,
-    int lm_count, float sigma_r, float sigma_b, float gate, float3 p0, Quat q0,
-    float3 p1, Quat q1, int use_packed, float& out0, float& out1) {
-    __shared__ float4 s_a[kObsChunk];
-    __shared__ float4 s_b[kObsChunk];
-    __shared__ float4 s_p[3 * kObsChunk];
+__device__ __forceinline__ void scalar_terms(const GateConsts& g, float3 p0, const Quat& qc0,
+                                             float3 p1, const Quat& qc1, const float4* s_a,
+                                             const float4* s_b, int cn, float2& acc) {
+    for (int k = 0; k < cn; ++k) {
+        const float4 a = s_a[k], b = s_b[k];
+        const int kind = __float_as_int(a.w);
+        obs_loglik(g, p0, qc0, a, b, kind, acc.x);
+        obs_loglik(g, p1, qc1, a, b, kind, acc.y);
+    }
+}
+
+// How weight_two forms its terms: by scalar arithmetic, packed, or packed for landmarks
+// that are not tame (see kTameCoord).
+enum WeightArith : int { ARITH_SCALAR = 0, ARITH_PACKED = 1, ARITH_PACKED_WILD = 2 };
+
+struct WeightPair {
+    float2 acc;
+    bool cart;  // every observation kept was Cartesian
+};
+
+// weight_two where the arithmetic is scalar, or a landmark or a pose of the block is not
+// tame: chunks with bearings then go by scalar arithmetic.  A function of its own, so the
+// packed loops carry nothing of it (a test and a branch in them cost 2 to 10 %).
+static __device__ __noinline__ WeightPair weight_two_general(
+    const CObservation* __restrict__ obs, int nobs, const float* __restrict__ lm, int lm_count,
+    float sigma_r, float sigma_b, float gate, float3 p0, Quat q0, float3 p1, Quat q1, int arith,
+    float4* s_a, float4* s_b, float4* s_p) {
     const GateConsts g = gate_consts(sigma_r, sigma_b, gate);
     const Quat qc0 = q_conjugate(q0), qc1 = q_conjugate(q1);
     const PackedPose pk = pack_pose(p0, qc0, p1, qc1);
-    const float2 ninv = make_float2(-g.inv2rr, -g.inv2rr);
-    float acc0 = 0.0f, acc1 = 0.0f;
-    bool cart = true;
+    WeightPair r{make_float2(0.0f, 0.0f), true};
     for (int c0 = 0; c0 < nobs; c0 += kObsChunk) {
         bool all_cart;
         __syncthreads();
         const int cn = stage_chunk(obs, lm, lm_count, c0, min(kObsChunk, nobs - c0),
                                    s_a, s_b, s_p, &all_cart);
+        r.cart = r.cart && all_cart;
+        if (all_cart && arith != ARITH_SCALAR)
+            packed_terms(pk, g, s_a, s_b, s_p, cn, r.acc);
+        else
+            scalar_terms(g, p0, qc0, p1, qc1, s_a, s_b, cn, r.acc);
+    }
+    return r;
+}
+
+// Gated log-likelihoods of two particles (p0,q0) and (p1,q1) against nobs
+// observations, staged kObsChunk at a time into shared memory (the whole
+// block takes part).  Packed or scalar, every path produces the reference's
+// roundings.  Returns whether every observation kept was Cartesian.
+__device__ __forceinline__ bool weight_two(
+    const CObservation* __restrict__ obs, int nobs, const float* __restrict__ lm,
+    int lm_count, float sigma_r, float sigma_b, float gate, float3 p0, Quat q0,
+    float3 p1, Quat q1, int arith, float& out0, float& out1) {
+    __shared__ float4 s_a[kObsChunk];
+    __shared__ float4 s_b[kObsChunk];
+    __shared__ float4 s_p[3 * kObsChunk];
+    const PackedPose pk = pack_pose(p0, q_conjugate(q0), p1, q_conjugate(q1));
+    if (__syncthreads_or(arith != ARITH_PACKED || !tame_pose(pk))) {
+        const WeightPair r = weight_two_general(obs, nobs, lm, lm_count, sigma_r, sigma_b, gate,
+                                                p0, q0, p1, q1, arith, s_a, s_b, s_p);
+        out0 = r.acc.x;
+        out1 = r.acc.y;
+        return r.cart;
+    }
+    const GateConsts g = gate_consts(sigma_r, sigma_b, gate);
+    const float2 ninv = make_float2(-g.inv2rr, -g.inv2rr);
+    float2 acc = make_float2(0.0f, 0.0f);
+    bool cart = true;
+    for (int c0 = 0; c0 < nobs; c0 += kObsChunk) {
+        bool all_cart;
+        if (c0) __syncthreads();
+        const int cn = stage_chunk(obs, lm, lm_count, c0, min(kObsChunk, nobs - c0),
+                                   s_a, s_b, s_p, &all_cart);
         cart = cart && all_cart;
-        if (!all_cart && use_packed) {
-            float2 acc = make_float2(acc0, acc1);
+        if (!all_cart) {
             packed_terms(pk, g, s_a, s_b, s_p, cn, acc);
-            acc0 = acc.x;
-            acc1 = acc.y;
-        } else if (all_cart && use_packed) {
-            float2 acc = make_float2(acc0, acc1);
-            if (gate > 0.0f) {
-#pragma unroll 2
-                for (int k = 0; k < cn; ++k) {
-                    const float2 r2 = packed_r2(pk, s_p[3 * k], s_p[3 * k + 1],
-                                                s_p[3 * k + 2]);
-                    const float2 t = __fmul2_rn(r2, ninv);
-                    const float a0 = (r2.x > g.cart_gate2) ? g.cart_out : t.x;
-                    const float a1 = (r2.y > g.cart_gate2) ? g.cart_out : t.y;
-                    acc = __fadd2_rn(acc, make_float2(a0, a1));
-                }
-            } else {
-#pragma unroll 2
-                for (int k = 0; k < cn; ++k) {
-                    const float2 r2 = packed_r2(pk, s_p[3 * k], s_p[3 * k + 1],
-                                                s_p[3 * k + 2]);
-                    // two roundings, as the reference (see cart_term)
-                    acc.x = __fadd_rn(acc.x, __fmul_rn(r2.x, ninv.x));
-                    acc.y = __fadd_rn(acc.y, __fmul_rn(r2.y, ninv.y));
-                }
-            }
-            acc0 = acc.x;
-            acc1 = acc.y;
-        } else if (all_cart && gate > 0.0f) {
+        } else if (gate > 0.0f) {
 #pragma unroll 2
             for (int k = 0; k < cn; ++k) {
-                const float4 a = s_a[k], b = s_b[k];
-                cart_term<true>(g, p0, qc0, a, b, acc0);
-                cart_term<true>(g, p1, qc1, a, b, acc1);
-            }
-        } else if (all_cart) {
-#pragma unroll 2
-            for (int k = 0; k < cn; ++k) {
-                const float4 a = s_a[k], b = s_b[k];
-                cart_term<false>(g, p0, qc0, a, b, acc0);
-                cart_term<false>(g, p1, qc1, a, b, acc1);
+                const float2 r2 = packed_r2(pk, s_p[3 * k], s_p[3 * k + 1],
+                                            s_p[3 * k + 2]);
+                const float2 t = __fmul2_rn(r2, ninv);
+                const float a0 = (r2.x > g.cart_gate2) ? g.cart_out : t.x;
+                const float a1 = (r2.y > g.cart_gate2) ? g.cart_out : t.y;
+                acc = __fadd2_rn(acc, make_float2(a0, a1));
             }
         } else {
+#pragma unroll 2
             for (int k = 0; k < cn; ++k) {
-                const float4 a = s_a[k], b = s_b[k];
-                const int kind = __float_as_int(a.w);
-                obs_loglik(g, p0, qc0, a, b, kind, acc0);
-                obs_loglik(g, p1, qc1, a, b, kind, acc1);
+                const float2 r2 = packed_r2(pk, s_p[3 * k], s_p[3 * k + 1],
+                                            s_p[3 * k + 2]);
+                // two roundings, as the reference's product and sum
+                acc.x = __fadd_rn(acc.x, __fmul_rn(r2.x, ninv.x));
+                acc.y = __fadd_rn(acc.y, __fmul_rn(r2.y, ninv.y));
             }
         }
     }
-    out0 = acc0;
-    out1 = acc1;
+    out0 = acc.x;
+    out1 = acc.y;
     return cart;
 }
 

@@ -258,6 +258,7 @@ struct PfHandle {
     float* d_lm = nullptr;
     int lm_count = 0;
     int lm_cap = 0;
+    bool lm_wild = false;  // a landmark of the table may not be tame (tame_landmark)
 
     // observations: device buffer + pinned staging ring
     CObservation* d_obs = nullptr;

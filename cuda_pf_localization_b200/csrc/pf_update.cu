@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kWThreads, 5)
              const CObservation* __restrict__ obs, int nobs,
              const float* __restrict__ lm, int lm_count, float sigma_r,
              float sigma_b, float gate, float* __restrict__ ll,
-             float2* part, unsigned* done, CycleCtl* ctl, int use_packed,
+             float2* part, unsigned* done, CycleCtl* ctl, int arith,
              const CycleArgs* ca, int block0) {
     pdl_wait();
     if (ca) {  // graph replay: this cycle's values
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(kWThreads, 5)
     }
     float acc0, acc1;
     const bool cart = weight_two(obs, nobs, lm, lm_count, sigma_r, sigma_b, gate, p0, q0, p1, q1,
-                                 use_packed, acc0, acc1);
+                                 arith, acc0, acc1);
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl->obs_cart = cart ? 1 : 0;
     if (v0) ll[i0] = acc0;
     if (v1) ll[i1] = acc1;
@@ -206,8 +206,8 @@ __device__ __forceinline__ float2 tile_softmax_partial(const float* s_ll, int co
 // Any observations: k_weight_marks' way with bearings, k_weight's arithmetic by four
 // groups of kWThreads threads, a 256-particle tile each at a time.  Sixteen warps an SM
 // where k_weight has twenty, and a block's tiles do not divide evenly: 1M x 64 / 256, one
-// bearing among them, 395 us against 315, every third one 556 and 478, all of them 880
-// and 752 (a particle a thread with scalar arithmetic on half of the block: 2.3 to 2.9
+// bearing among them, 389 us against 314, every third one 542 and 469, all of them 846
+// and 741 (a particle a thread with scalar arithmetic on half of the block: 2.3 to 2.9
 // times k_weight's).
 template <bool kPredict>
 __device__ __noinline__ void weight_tiles(MarksSmem& sm, const Planes& s, int n, uint64_t seed,
@@ -237,9 +237,23 @@ __device__ __noinline__ void weight_tiles(MarksSmem& sm, const Planes& s, int n,
     const unsigned kept = __ballot_sync(~0u, keep);
     int at = __popc(kept & ((1u << lane) - 1u));
     for (int k = 0; k < warp; ++k) at += sm.warp_count[k];  // left by marks_build
-    if (keep) stage_one(o, lm, at, s_a, s_b, s_p);
-    const int cn = sm.kept;
-    __syncthreads();
+    bool is_wild = false;
+    if (keep) {
+        stage_one(o, lm, at, s_a, s_b, s_p);
+        const float4 a = s_a[at];
+        is_wild = !tame_landmark(a.x, a.y, a.z);
+    }
+    // k_weight's chunks: where one starts, whether it has bearings, and wild landmarks
+    constexpr int kChunks = kMObs / kObsChunk;
+    int start[kChunks + 1] = {0};
+    bool mixed[kChunks];
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c) {
+        const bool mine = keep && tid / kObsChunk == c;
+        start[c + 1] = start[c] + __syncthreads_count(mine);
+        mixed[c] = __syncthreads_or(mine && o.mode != 0);
+    }
+    const bool wild = __syncthreads_or(is_wild);
     for (int tile = blockIdx.x + group * gridDim.x; (long long)tile * kMTile < n;
          tile += kGroups * gridDim.x) {
         const int i0 = tile * kMTile + t;
@@ -260,7 +274,16 @@ __device__ __noinline__ void weight_tiles(MarksSmem& sm, const Planes& s, int n,
         }
         const PackedPose pk = pack_pose(p[0], q_conjugate(q[0]), p[1], q_conjugate(q[1]));
         float2 acc = make_float2(0.f, 0.f);
-        packed_terms(pk, g, s_a, s_b, s_p, cn, acc);
+        const bool tame = !wild && tame_pose(pk);
+#pragma unroll 1
+        for (int c = 0; c < kChunks; ++c) {
+            const int at = start[c], cn = start[c + 1] - at;
+            if (mixed[c] && !tame)
+                scalar_terms(g, p[0], q_conjugate(q[0]), p[1], q_conjugate(q[1]), s_a + at,
+                             s_b + at, cn, acc);
+            else
+                packed_terms(pk, g, s_a + at, s_b + at, s_p + 3 * at, cn, acc);
+        }
         if (i0 < n) ll[i0] = acc.x;
         if (i0 + kWThreads < n) ll[i0 + kWThreads] = acc.y;
         s_ll[t] = acc.x;
@@ -461,6 +484,10 @@ bool weight_by_marks(const PfHandle* h, int nobs, bool cart) {
            (long long)h->n * (nobs - h->lm_count) >= 16000000;
 }
 
+static int weight_arith(const PfHandle* h) {
+    return h->weight_variant ? ARITH_SCALAR : h->lm_wild ? ARITH_PACKED_WILD : ARITH_PACKED;
+}
+
 int launch_reinit(PfHandle* h, const float p0[3], const float q0[4],
                   const float pstd[3], const float rstd[3]) {
     const int grid = ceil_div(h->n, kThreads);
@@ -509,12 +536,12 @@ int launch_weight(PfHandle* h, const PredictArgs& pa, const CObservation* d_obs,
         PFB_CK(launch_pdl(k_weight<true, false>, grid, kWThreads, 0, h->stream, plane_set(h),
                           h->n, h->seed, pa, d_obs, nobs, h->d_lm, h->lm_count,
                           sigma_r, sigma_b, gate, h->d_ll, part, h->d_done + 0,
-                          h->d_ctl, h->weight_variant == 0 ? 1 : 0, dargs, 0));
+                          h->d_ctl, weight_arith(h), dargs, 0));
     } else {
         PFB_CK(launch_pdl(k_weight<false, false>, grid, kWThreads, 0, h->stream, plane_set(h),
                           h->n, h->seed, pa, d_obs, nobs, h->d_lm, h->lm_count,
                           sigma_r, sigma_b, gate, h->d_ll, part, h->d_done + 0,
-                          h->d_ctl, h->weight_variant == 0 ? 1 : 0, dargs, 0));
+                          h->d_ctl, weight_arith(h), dargs, 0));
     }
     PFB_KL();
     h->prefix_valid = false;
@@ -537,7 +564,7 @@ int launch_weight_shard(PfHandle* h, const PredictArgs& pa, const CObservation* 
     PFB_CK(launch_pdl(k_weight<true, true>, grid, kWThreads, 0, h->stream, plane_set(h), h->n,
                       h->seed, pa, d_obs, nobs, h->d_lm, h->lm_count, sigma_r, sigma_b, gate,
                       h->d_ll, part, h->d_done + 0, h->d_ctl,
-                      h->weight_variant == 0 ? 1 : 0, (const CycleArgs*)nullptr, block0));
+                      weight_arith(h), (const CycleArgs*)nullptr, block0));
     PFB_KL();
     h->prefix_valid = false;
     return 0;
