@@ -228,9 +228,8 @@ __global__ void __launch_bounds__(kWThreads, 6)
         return;
     }
     float acc0, acc1;
-    weight_two(obs + in.obs_off, nobs, lm + 3 * (size_t)fl.lm_off, fl.lm_count,
-               fl.sigma_r, fl.sigma_b, fl.gate, p0, q0, p1, q1, arith, acc0,
-               acc1);
+    weight_two<false>(obs + in.obs_off, nobs, lm + 3 * (size_t)fl.lm_off, fl.lm_count,
+                      fl.sigma_r, fl.sigma_b, fl.gate, p0, q0, p1, q1, arith, acc0, acc1);
     float* ll = A.ll + fl.off;
     if (v0) ll[i0] = acc0;
     if (v1) ll[i1] = acc1;
@@ -576,9 +575,9 @@ __global__ void __launch_bounds__(kThreads, 3)
 // are already running when it looks back).  Source j writes j at the first
 // output of its run and at every gather-tile boundary inside it (runs are
 // disjoint, so no two sources write the same marker); k_b_gather copies.  Its
-// blocks mostly wait (the look-back, FP64 chains): four per SM (64 registers) where
-// 72 registers let three run took a 128-filter cycle of 4.7M particles from 515 to
-// 507 us; five and six were slower.
+// blocks mostly wait (the look-back, FP64 chains): four per SM (64 registers, a spill
+// of 32 bytes) where 72 registers let three run took a 128-filter cycle of 4.7M
+// particles from 515 to 507 us; five and six were slower.
 __global__ void __launch_bounds__(kThreads, 4)
     k_b_resample(Arena A, const BFilter* __restrict__ F, const BTile* __restrict__ T,
                  BCtl* C, BGlobal* G, unsigned* flags, uint64_t* vals) {
@@ -886,10 +885,11 @@ __global__ void k_b_inject_apply(Arena A, const BFilter* __restrict__ F,
 }
 
 // Commits every filter's resample and readies the batch for the next one; then the
-// estimate sums of a filter that resampled, without a pass over the new cloud: its gather tiles' sums in tile order, plus wd times the
-// injection's position changes in draw order; then the Markley mean and the
-// f32 means of the covariance pass, as the estimate pass's last tile leaves
-// them.  One block per filter; the others take the estimate pass.
+// estimate sums of a filter that resampled, without a pass over the new cloud: its
+// gather tiles' sums in tile order, plus wd times the injection's position changes in
+// draw order; then the Markley mean and the f32 means of the covariance pass, as the
+// estimate pass's last tile leaves them.  One block per filter; the others take the
+// estimate pass.
 __global__ void __launch_bounds__(kThreads)
     k_b_est_src(const BFilter* __restrict__ F, BCtl* C, BGlobal* G,
                 const double* gpart, const double* icorr) {

@@ -325,6 +325,24 @@ __device__ __forceinline__ int stage_chunk(const CObservation* __restrict__ obs,
     return total;
 }
 
+// Gated Cartesian term of the reference (pf_kernels.cu:247-252) for the
+// specialised all-Cartesian loop; gate > 0 is hoisted out as kGated.
+template <bool kGated>
+__device__ __forceinline__ void cart_term(const GateConsts& g, float3 p,
+                                          const Quat& qc, float4 a, float4 b,
+                                          float& acc) {
+    float3 d = make_float3(a.x - p.x, a.y - p.y, a.z - p.z);
+    float3 pred = q_rotate(qc, d);
+    const float ex = pred.x - b.x, ey = pred.y - b.y, ez = pred.z - b.z;
+    const float r2 = sq3(ex, ey, ez);
+    // The reference rounds the product and the sum separately in both the
+    // gated and the ungated case.
+    if (kGated)
+        acc = __fadd_rn(acc, (r2 > g.cart_gate2) ? g.cart_out : __fmul_rn(-r2, g.inv2rr));
+    else
+        acc = __fadd_rn(acc, __fmul_rn(-r2, g.inv2rr));
+}
+
 // ---------------------------------------------------------- packed path
 // The Cartesian term evaluated for two particles at once with packed f32x2
 // arithmetic.  nvcc compiles the reference expression (q_rotate + squared
@@ -617,9 +635,8 @@ struct WeightPair {
     bool cart;  // every observation kept was Cartesian
 };
 
-// weight_two where the arithmetic is scalar, or a landmark or a pose of the block is not
-// tame: chunks with bearings then go by scalar arithmetic.  A function of its own, so the
-// packed loops carry nothing of it (a test and a branch in them cost 2 to 10 %).
+// weight_two<true> where the arithmetic is scalar, or a landmark or a pose of the block
+// is not tame: chunks with bearings then go by scalar arithmetic.
 static __device__ __noinline__ WeightPair weight_two_general(
     const CObservation* __restrict__ obs, int nobs, const float* __restrict__ lm, int lm_count,
     float sigma_r, float sigma_b, float gate, float3 p0, Quat q0, float3 p1, Quat q1, int arith,
@@ -646,6 +663,14 @@ static __device__ __noinline__ WeightPair weight_two_general(
 // observations, staged kObsChunk at a time into shared memory (the whole
 // block takes part).  Packed or scalar, every path produces the reference's
 // roundings.  Returns whether every observation kept was Cartesian.
+// kApart: the scalar arithmetic is a call of its own, and poses that are not tame take
+// it (the single filter: 500k x 150 bearings 238 -> 235.5 us, 300k x 200 mixed 121.4 ->
+// 119.1, 1M x 256 Cartesian 271.3 -> 272.3).  Else it stands beside the packed
+// arithmetic, and only landmarks are looked at (the batch, whose Cartesian cycles lost
+// 2 % with a call; its poses come from priors and odometry, which would have to be near
+// the largest floats themselves).  A test and a branch in the packed loops cost 2 to
+// 10 %.
+template <bool kApart>
 __device__ __forceinline__ bool weight_two(
     const CObservation* __restrict__ obs, int nobs, const float* __restrict__ lm,
     int lm_count, float sigma_r, float sigma_b, float gate, float3 p0, Quat q0,
@@ -653,49 +678,80 @@ __device__ __forceinline__ bool weight_two(
     __shared__ float4 s_a[kObsChunk];
     __shared__ float4 s_b[kObsChunk];
     __shared__ float4 s_p[3 * kObsChunk];
-    const PackedPose pk = pack_pose(p0, q_conjugate(q0), p1, q_conjugate(q1));
-    if (__syncthreads_or(arith != ARITH_PACKED || !tame_pose(pk))) {
+    const GateConsts g = gate_consts(sigma_r, sigma_b, gate);
+    const Quat qc0 = q_conjugate(q0), qc1 = q_conjugate(q1);
+    const PackedPose pk = pack_pose(p0, qc0, p1, qc1);
+    if (kApart && __syncthreads_or(arith != ARITH_PACKED || !tame_pose(pk))) {
         const WeightPair r = weight_two_general(obs, nobs, lm, lm_count, sigma_r, sigma_b, gate,
                                                 p0, q0, p1, q1, arith, s_a, s_b, s_p);
         out0 = r.acc.x;
         out1 = r.acc.y;
         return r.cart;
     }
-    const GateConsts g = gate_consts(sigma_r, sigma_b, gate);
     const float2 ninv = make_float2(-g.inv2rr, -g.inv2rr);
-    float2 acc = make_float2(0.0f, 0.0f);
+    float acc0 = 0.0f, acc1 = 0.0f;
     bool cart = true;
     for (int c0 = 0; c0 < nobs; c0 += kObsChunk) {
         bool all_cart;
-        if (c0) __syncthreads();
+        __syncthreads();
         const int cn = stage_chunk(obs, lm, lm_count, c0, min(kObsChunk, nobs - c0),
                                    s_a, s_b, s_p, &all_cart);
         cart = cart && all_cart;
-        if (!all_cart) {
+        if (!all_cart && (kApart || arith == ARITH_PACKED)) {
+            float2 acc = make_float2(acc0, acc1);
             packed_terms(pk, g, s_a, s_b, s_p, cn, acc);
-        } else if (gate > 0.0f) {
+            acc0 = acc.x;
+            acc1 = acc.y;
+        } else if (kApart || (all_cart && arith != ARITH_SCALAR)) {
+            float2 acc = make_float2(acc0, acc1);
+            if (gate > 0.0f) {
+#pragma unroll 2
+                for (int k = 0; k < cn; ++k) {
+                    const float2 r2 = packed_r2(pk, s_p[3 * k], s_p[3 * k + 1],
+                                                s_p[3 * k + 2]);
+                    const float2 t = __fmul2_rn(r2, ninv);
+                    const float a0 = (r2.x > g.cart_gate2) ? g.cart_out : t.x;
+                    const float a1 = (r2.y > g.cart_gate2) ? g.cart_out : t.y;
+                    acc = __fadd2_rn(acc, make_float2(a0, a1));
+                }
+            } else {
+#pragma unroll 2
+                for (int k = 0; k < cn; ++k) {
+                    const float2 r2 = packed_r2(pk, s_p[3 * k], s_p[3 * k + 1],
+                                                s_p[3 * k + 2]);
+                    // two roundings, as the reference (see cart_term)
+                    acc.x = __fadd_rn(acc.x, __fmul_rn(r2.x, ninv.x));
+                    acc.y = __fadd_rn(acc.y, __fmul_rn(r2.y, ninv.y));
+                }
+            }
+            acc0 = acc.x;
+            acc1 = acc.y;
+        } else if (all_cart && gate > 0.0f) {  // (one scalar loop for all: the batch's packed
+                                               // Cartesian cycles 4 % slower)
 #pragma unroll 2
             for (int k = 0; k < cn; ++k) {
-                const float2 r2 = packed_r2(pk, s_p[3 * k], s_p[3 * k + 1],
-                                            s_p[3 * k + 2]);
-                const float2 t = __fmul2_rn(r2, ninv);
-                const float a0 = (r2.x > g.cart_gate2) ? g.cart_out : t.x;
-                const float a1 = (r2.y > g.cart_gate2) ? g.cart_out : t.y;
-                acc = __fadd2_rn(acc, make_float2(a0, a1));
+                const float4 a = s_a[k], b = s_b[k];
+                cart_term<true>(g, p0, qc0, a, b, acc0);
+                cart_term<true>(g, p1, qc1, a, b, acc1);
+            }
+        } else if (all_cart) {
+#pragma unroll 2
+            for (int k = 0; k < cn; ++k) {
+                const float4 a = s_a[k], b = s_b[k];
+                cart_term<false>(g, p0, qc0, a, b, acc0);
+                cart_term<false>(g, p1, qc1, a, b, acc1);
             }
         } else {
-#pragma unroll 2
             for (int k = 0; k < cn; ++k) {
-                const float2 r2 = packed_r2(pk, s_p[3 * k], s_p[3 * k + 1],
-                                            s_p[3 * k + 2]);
-                // two roundings, as the reference's product and sum
-                acc.x = __fadd_rn(acc.x, __fmul_rn(r2.x, ninv.x));
-                acc.y = __fadd_rn(acc.y, __fmul_rn(r2.y, ninv.y));
+                const float4 a = s_a[k], b = s_b[k];
+                const int kind = __float_as_int(a.w);
+                obs_loglik(g, p0, qc0, a, b, kind, acc0);
+                obs_loglik(g, p1, qc1, a, b, kind, acc1);
             }
         }
     }
-    out0 = acc.x;
-    out1 = acc.y;
+    out0 = acc0;
+    out1 = acc1;
     return cart;
 }
 

@@ -165,8 +165,8 @@ __global__ void __launch_bounds__(kWThreads, 5)
         }
     }
     float acc0, acc1;
-    const bool cart = weight_two(obs, nobs, lm, lm_count, sigma_r, sigma_b, gate, p0, q0, p1, q1,
-                                 arith, acc0, acc1);
+    const bool cart = weight_two<true>(obs, nobs, lm, lm_count, sigma_r, sigma_b, gate, p0, q0,
+                                       p1, q1, arith, acc0, acc1);
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl->obs_cart = cart ? 1 : 0;
     if (v0) ll[i0] = acc0;
     if (v1) ll[i1] = acc1;
