@@ -75,7 +75,7 @@ constexpr uint32_t kWaitLimit = 1u << 24;
 enum Epi : int {
     EPI_RELU_BF16 = 0,   // bf16 relu(acc + bias), row-major and transposed
     EPI_BIAS_F32 = 1,    // f32 acc + bias, row-major
-    EPI_DRELU_BF16 = 2,  // bf16 acc * (mask > 0), row-major and transposed
+    EPI_DRELU_BF16 = 2,  // bf16 acc gated by the bits of relu', row-major and transposed
     EPI_F32 = 3,         // f32 acc * scale, row-major
 };
 
