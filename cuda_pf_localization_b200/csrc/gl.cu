@@ -894,11 +894,13 @@ int ensure_scan(GlHandle* h, const float* scan, int nrays) {
 // grid leaves room for fewer than kMinSmemWarps it stays in global memory; so it does
 // where a ray could take more than 8192 steps, which the shared-memory stepping does
 // not count.  Its cells then come through L1, which has what the slots leave of the
-// SM's memory: two blocks of 24 warps where their slots fit, else one of 24 and not
-// two of fewer (20 000 hypotheses on 600 x 600 cells, 600 rays: 4.7 ms and 9.0 with
-// two blocks, 1000 rays 8.0 and 12.0).
+// SM's memory: two blocks of 24 warps where their slots fit, else one of 24 (23 for the
+// last ray counts) and not two of fewer (20 000 hypotheses on 600 x 600 cells: 4.3 ms and
+// 9.0 with two blocks at 600 rays, 7.2 and 12.0 at 1000; 7.7 with 23 warps at 1040, 12.2
+// with 24).
 constexpr int kSmBytes = 233472 - 2 * 1088;  // of an SM, less what each block reserves
 constexpr int kMaxSlotBytes = 200 * 1024;    // ray slots of 24 warps and the scan
+constexpr int kL1SlotBytes = 196 * 1024 - 1088;  // as much of it as leaves L1 60 KB
 constexpr int kMinSmemWarps = 10;
 
 struct ScorePlan {
@@ -926,7 +928,7 @@ bool score_plan(const GlHandle* h, int nrays, int nscan, ScorePlan* p) {
         p->warps = p->per_sm == 2 ? pair : solo;
         p->bytes = (size_t)(grid + scan + slot * p->warps);
     } else {
-        p->warps = kPairThreads / 32;
+        p->warps = (int)std::min<long long>(kPairThreads / 32, (kL1SlotBytes - scan) / slot);
         p->bytes = (size_t)(scan + slot * p->warps);
         p->per_sm = 2 * (long long)p->bytes <= kSmBytes ? 2 : 1;
     }
